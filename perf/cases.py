@@ -304,3 +304,54 @@ def tolerance(case):
     if case["kind"] == "mlp1":
         return {"rel": 6e-4}
     return {"rel": 2e-6, "max": 2e-5}
+
+
+# ------------------------------------------------------------------------------- exact
+def _dequantised(w):
+    """Rows of a packed weight in 64 bits, a block of rows at a time: (first row, values)."""
+    M, K = w.rec.M, w.rec.K
+    for r0 in range(0, M, 1024):
+        rows = min(1024, M - r0)
+        t = slice(r0 // 16, (r0 + rows) // 16)
+        if isinstance(w, _Weight8):
+            s, z = w.scales[t].double(), 0.0
+            q = w.codes[t].double()
+        else:
+            word = w.scales[t].to(torch.int32)
+            s = (word & 0xFFF0).to(torch.int16).view(torch.float16).double()
+            z = (((word & 15) ^ 8) - 8).double().transpose(1, 2).reshape(rows, -1, 1)
+            c = w.codes[t].to(torch.int32)
+            q = ((torch.stack((c & 15, c >> 4), -1) ^ 8) - 8).double()
+        q = q.reshape(rows // 16, K // 32, 16, 32).transpose(1, 2).reshape(rows, K)
+        s = s.transpose(1, 2).reshape(rows, -1, 1)
+        yield r0, ((q.reshape(rows, s.shape[1], -1) - z) * s).reshape(rows, K)
+
+
+def _quantised(x, block, levels):
+    """Rows as their codes stand for them: one scale, the largest magnitude / levels, per block. The
+    scale and the code are what fp32 gives (they are data to the sums), the product is exact."""
+    v = x.float().reshape(x.shape[0], -1, block)
+    top = v.abs().amax(2, keepdim=True)
+    s = torch.where(top > 0, top / levels, torch.ones_like(top))
+    return (torch.round(v / s).clamp(-levels, levels).double() * s.double()).reshape(x.shape)
+
+
+def _project(w, xq):
+    y = torch.empty(xq.shape[0], w.rec.M, dtype=torch.float64, device="cuda")
+    for r0, v in _dequantised(w):
+        y[:, r0:r0 + v.shape[0]] = xq @ v.T
+    return y
+
+
+def exact(case, seed):
+    s = prepare(case, seed)
+    if case["kind"] == "mlp1":
+        x = s["x"].double()
+        xn = x / torch.sqrt((x * x).mean() + 1e-6) * (1.0 + s["norm"].double())
+        g, u = (_project(w, _quantised(xn[None], 32, 127))[0] for w in (s["gate"], s["up"]))
+        h = g / (1.0 + torch.exp(-g)) * u
+        return [xn, g, u, h, _project(s["down"], _quantised(h[None], 32, 127))[0] + x]
+    act = case.get("act", "block")
+    block, levels = (64, 7) if act == "int4" else ((case["K"], 127) if act.startswith("token") else (32, 127))
+    xq = _quantised(s["x"], block, levels)
+    return [_project(w, xq) for w in s["w"]]
