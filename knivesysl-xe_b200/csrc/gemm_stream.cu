@@ -463,7 +463,7 @@ __device__ unsigned long long g_ring_trace[1024 * 8];
 #define RING_STAMP(i)
 #define RING_STAMP_END()
 #endif
-// NTG: 8-token groups a warp carries per tile (1, 2, 4 or 8): the tile's A fragments, scale
+// NTG: 8-token groups a warp carries per tile (1 to 8): the tile's A fragments, scale
 // words and ring traffic are paid once for all of them; the staged activations of group g
 // follow those of group g - 1 (`gstride` bytes apart).
 template <bool PAIR, int kRNS, int MAXW, bool PT, int NTG = 1>
@@ -1019,7 +1019,14 @@ bool ring_plan_ntg(const GemmArgs &a, int ntg, RingPlan &p) {
     return p.smem <= kSmemLimit;
 }
 // The widest plan that fits: all of a call's tokens on one warp (weights and their unpacking
-// paid once), else windows of 32, 16 or 8 tokens on CTA columns.
+// paid once), else windows of 32, 16 or 8 tokens on CTA columns. In per-token mode every number of
+// token groups has an instantiation; before 3, 5, 6 and 7 had one, 24 tokens ran as three windows
+// and 40 as five, each unpacking all weights (5120 x 17408 K32, us with staging: 24 tokens 43.5 -> 32.8,
+// 40: 122 -> 50, 48: 71 -> 58, 56: 125 -> 65). Two exceptions keep the windows: the reference's
+// arithmetic, whose split rule leaves few tasks per call (24 tokens 42.0 against 43.8 us on that
+// shape, 48 tokens 19.6 against 24.7 on 2 x 1024 x 5120), and 48 tokens whose splits are shorter than
+// four k-tiles, where the ordered reduction of the wider partials outweighs the unpacking
+// (3 x 1040 x 1088: 27.0 against 30.3 us).
 bool ring_plan(const GemmArgs &a, RingPlan &p) {
     if (a.T < 8 || a.T > 64 || (a.T % 8) || a.dump) return false;
     if (a.x && (a.T != 8 || a.mode)) return false;   // the fused quantiser serves one window
@@ -1030,8 +1037,13 @@ bool ring_plan(const GemmArgs &a, RingPlan &p) {
         if (g_num_sms <= 0) g_num_sms = 148;
     }
     const int tg = a.T / 8;
-    for (int ntg = 8; ntg >= 1; ntg >>= 1)
-        if (tg % ntg == 0 && (ntg == 1 || !a.npeer) && ring_plan_ntg(a, ntg, p)) return true;
+    const bool short_splits = (a.K >> 5) < 4 * a.max_splits;
+    auto has_kernel = [&](int ntg) {
+        if (!(ntg & (ntg - 1))) return true;                 // 8, 4, 2, 1
+        return a.mode && !(ntg == 6 && short_splits);
+    };
+    for (int ntg = 8; ntg >= 1; --ntg)
+        if (tg % ntg == 0 && has_kernel(ntg) && (ntg == 1 || !a.npeer) && ring_plan_ntg(a, ntg, p)) return true;
     return false;
 }
 
@@ -1048,14 +1060,14 @@ bool launch_ring(const GemmArgs &a) {
     if (S > 1) ensure_scratch((size_t)plan.nwin * groups * S * 128 * plan.ntg, plan.nwin * groups);
     auto go = [&](auto kernel) {
         // every instantiation has the same function type, so remember them by address
-        static const void *done[64];
+        static const void *done[96];
         static int ndone = 0;
         bool seen = false;
         for (int i = 0; i < ndone; ++i) seen = seen || done[i] == (const void *)kernel;
         if (!seen) {
             TQ_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                           (int)kSmemLimit));
-            if (ndone < 64) done[ndone++] = (const void *)kernel;
+            if (ndone < 96) done[ndone++] = (const void *)kernel;
         }
         launch_pdl(kernel, dim3(grid, plan.nwin), dim3(nw * 32), smem, a, g_scratch.part, g_scratch.count);
     };
@@ -1064,6 +1076,14 @@ bool launch_ring(const GemmArgs &a) {
         if (plan.ntg == 8) go(gemm_w4a8_ring_kernel<P, 3, 20, Q, 8>);
         else if (plan.ntg == 4) go(gemm_w4a8_ring_kernel<P, 3, 20, Q, 4>);
         else if (plan.ntg == 2) go(gemm_w4a8_ring_kernel<P, 3, 20, Q, 2>);
+        else if (plan.ntg > 1) {
+            if constexpr (Q) {                               // per-token mode only
+                if (plan.ntg == 7) go(gemm_w4a8_ring_kernel<P, 3, 20, true, 7>);
+                else if (plan.ntg == 6) go(gemm_w4a8_ring_kernel<P, 3, 20, true, 6>);
+                else if (plan.ntg == 5) go(gemm_w4a8_ring_kernel<P, 3, 20, true, 5>);
+                else go(gemm_w4a8_ring_kernel<P, 3, 20, true, 3>);
+            }
+        }
         else if (ns == 2) go(gemm_w4a8_ring_kernel<P, 2, kRW, Q>);
         else if (ns == 3) go(gemm_w4a8_ring_kernel<P, 3, kRW, Q>);
         else if (nw <= 20) go(gemm_w4a8_ring_kernel<P, 4, 20, Q>);
