@@ -1,7 +1,7 @@
 """Prefill GEMM (csrc/gemm_tc.cu): every tile width it chooses between, and a caller whose code sums
 are not the sums of its codes.
 
-The kernel takes 64, 128, 192 or 256 tokens a tile, by the rounds that M / 128 row blocks x token
+The kernel takes 128, 192 or 256 tokens a tile, by the rounds that M / 128 row blocks x token
 blocks make on 148 SMs; the sizes below select each of them, with a ragged last block, a full one
 and more than one round of tiles. Zero points are taken off the weights before the dot, so that
 z * asum enters as z * sum(codes); an asum that is something else takes a kernel of its own. Every
@@ -11,11 +11,11 @@ import numpy as np
 import pytest
 
 SIZES = [
-    (128, 64, 136),        # 64 a tile, one row block, last block of 8 tokens
-    (5120, 128, 136),      # 64 a tile, 120 tiles
+    (128, 64, 136),        # one row block
+    (5120, 128, 136),      # few row blocks
     (9472, 128, 248),      # 128 a tile, exactly one round
     (10240, 128, 136),     # 192 a tile, one ragged block
-    (128, 192, 1000),      # 64 a tile, three steps: an odd number of slot uses
+    (128, 192, 1000),      # one row block, three steps: an odd number of slot uses
     (17408, 128, 256),     # 256 a tile, one full block
     (17408, 64, 320),      # several rounds: a CTA walks from tile to tile
 ]
