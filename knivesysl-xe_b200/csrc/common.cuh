@@ -319,9 +319,21 @@ inline void launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, 
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// A CTA's shared memory may be accessed by the others only once it has started, which nothing but a
+// cluster barrier shows: every thread calls cluster_arrive() at kernel entry and cluster_wait()
+// before the first store, so that the barrier's latency lies under the loads in between. The token
+// is what a store into a peer asks for.
+struct ClusterStarted {};
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ ClusterStarted cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    return {};
+}
 // Stores v at the address that `local` (a shared-memory address of this CTA) has in CTA
 // `rank` of the cluster.
-__device__ __forceinline__ void st_cluster_f32(uint32_t local, uint32_t rank, float v) {
+__device__ __forceinline__ void st_cluster_f32(ClusterStarted, uint32_t local, uint32_t rank, float v) {
     uint32_t remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");

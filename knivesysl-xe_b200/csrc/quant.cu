@@ -178,6 +178,7 @@ rmsnorm_quant_cluster_kernel(float *__restrict__ out, const float *__restrict__ 
                              int8_t *__restrict__ q, int8_t *__restrict__ qp, float *__restrict__ scale,
                              int32_t *__restrict__ sum16, int32_t *__restrict__ sum32) {
     pdl_trigger();
+    cluster_arrive();
     pdl_wait();
     __shared__ float wsum[4][8];
     __shared__ float part[32];
@@ -198,12 +199,13 @@ rmsnorm_quant_cluster_kernel(float *__restrict__ out, const float *__restrict__ 
         if (lane == 0) wsum[u][warp] = s;
     }
     __syncthreads();
+    const ClusterStarted peers = cluster_wait();
     if ((int)threadIdx.x < 4 * C) {                  // block u's sum, stored into CTA `rank`
         const int u = threadIdx.x / C, rank = threadIdx.x % C;
         float t = 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) t = __fadd_rn(t, wsum[u][k]);
-        st_cluster_f32((uint32_t)__cvta_generic_to_shared(&part[u * C + c]), (uint32_t)rank, t);
+        st_cluster_f32(peers, (uint32_t)__cvta_generic_to_shared(&part[u * C + c]), (uint32_t)rank, t);
     }
     cluster_sync_all();
     float sum_sq = 0.0f;
@@ -587,6 +589,7 @@ quant_chunk_pertoken_cluster_kernel(const ClusterSrc src, int K, int T,
                                     int32_t *__restrict__ asum, float *__restrict__ as_tok,
                                     const SyncArgs sync) {
     pdl_trigger();
+    cluster_arrive();
     pdl_wait();
     exchange_sync(sync);
     __shared__ float wmax[8];
@@ -637,9 +640,10 @@ quant_chunk_pertoken_cluster_kernel(const ClusterSrc src, int K, int T,
     m = warp_max(m);
     if (lane == 0) wmax[warp] = m;
     __syncthreads();
+    const ClusterStarted peers = cluster_wait();
     if (warp == 0) {
         const float t = warp_max(lane < 8 ? wmax[lane] : -INFINITY);
-        if (lane < C) st_cluster_f32((uint32_t)__cvta_generic_to_shared(&cmax[c]), (uint32_t)lane, t);
+        if (lane < C) st_cluster_f32(peers, (uint32_t)__cvta_generic_to_shared(&cmax[c]), (uint32_t)lane, t);
     }
     cluster_sync_all();
     float t = cmax[0];
@@ -683,6 +687,7 @@ quant_s8_rowscale_cluster_kernel(const float *__restrict__ x, const float *__res
                                  int8_t *__restrict__ qp, float *__restrict__ scale,
                                  int32_t *__restrict__ sum16, int32_t *__restrict__ sum32) {
     pdl_trigger();
+    cluster_arrive();
     pdl_wait();
     __shared__ float wmax[8];
     __shared__ float cmax[8];
@@ -710,9 +715,10 @@ quant_s8_rowscale_cluster_kernel(const float *__restrict__ x, const float *__res
     m = warp_max(m);
     if (lane == 0) wmax[warp] = m;
     __syncthreads();
+    const ClusterStarted peers = cluster_wait();
     if (warp == 0) {
         const float t = warp_max(lane < 8 ? wmax[lane] : -INFINITY);
-        if (lane < C) st_cluster_f32((uint32_t)__cvta_generic_to_shared(&cmax[c]), (uint32_t)lane, t);
+        if (lane < C) st_cluster_f32(peers, (uint32_t)__cvta_generic_to_shared(&cmax[c]), (uint32_t)lane, t);
     }
     cluster_sync_all();
     float t = cmax[0];
