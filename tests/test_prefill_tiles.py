@@ -3,7 +3,9 @@ are not the sums of its codes.
 
 The kernel takes 128, 192 or 256 tokens a tile, by the rounds that M / 128 row blocks x token
 blocks make on 148 SMs; the sizes below select each of them, with a ragged last block, a full one
-and more than one round of tiles. Zero points are taken off the weights before the dot, so that
+and more than one round of tiles. A tile is K / 64 steps; the step slots (6, 5 and 4 at the three
+widths) and the accumulator buffers are used in turn, so REFILL goes through every slot at least
+twice, with odd step counts, within one tile and from tile to tile. Zero points are taken off the weights before the dot, so that
 z * asum enters as z * sum(codes); an asum that is something else takes a kernel of its own. Every
 output word is compared with the oracle, which reads asum as given: all terms up to the promote are
 integers below 2^24 in either association, so no tolerance is needed."""
@@ -11,14 +13,27 @@ import numpy as np
 import pytest
 
 SIZES = [
-    (128, 64, 136),        # one row block
     (5120, 128, 136),      # few row blocks
     (9472, 128, 248),      # 128 a tile, exactly one round
     (10240, 128, 136),     # 192 a tile, one ragged block
-    (128, 192, 1000),      # one row block, three steps: an odd number of slot uses
     (17408, 128, 256),     # 256 a tile, one full block
     (17408, 64, 320),      # several rounds: a CTA walks from tile to tile
 ]
+# one row block; block scales need 2048 tokens and more there, or the call is split and goes elsewhere
+ONE_ROW_BLOCK = {
+    "block": [(128, 64, 2048), (128, 192, 2056)],
+    "other": [(128, 64, 136), (128, 192, 1000)],
+}
+REFILL = [
+    (1024, 1600, 256),     # 128 a tile, 25 steps: every slot refilled four times
+    (19200, 320, 128),     # 128 a tile, two tiles of 5 steps on a CTA
+    (9600, 1088, 136),     # 192 a tile, 17 steps on 5 slots
+    (20480, 320, 136),     # 192 a tile, two tiles of 5 steps on a CTA
+    (9600, 832, 200),      # 256 a tile, 13 steps on 4 slots
+    (28544, 320, 200),     # 256 a tile, two tiles of 5 steps on a CTA
+]
+MODES = ["block_k32", "block_k64", "token_k32", "token_k64", "w4a4"]
+CASES = [(m, s) for m in MODES for s in SIZES + ONE_ROW_BLOCK["block" if m.startswith("block") else "other"] + REFILL]
 
 
 def _buf(pkg, a):
@@ -27,12 +42,12 @@ def _buf(pkg, a):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("wrong_sums", [False, True])
-@pytest.mark.parametrize("M,K,T", SIZES)
-@pytest.mark.parametrize("mode", ["block_k32", "block_k64", "token_k32", "token_k64", "w4a4"])
-def test_prefill_tile_widths(lib, pkg, orc, wl, mode, M, K, T, wrong_sums):
+@pytest.mark.parametrize("mode,size", CASES, ids=lambda v: v if isinstance(v, str) else "x".join(map(str, v)))
+def test_prefill_tile_widths(lib, pkg, orc, wl, mode, size, wrong_sums):
+    M, K, T = size
     ksh = 0 if mode.endswith("k32") else 1
-    if mode.startswith("block") and lib.qwn_choose_gemm_splits(M // 16, T // 8, K // 32) != 1:
-        pytest.skip("the call is split: not the prefill kernel's")
+    if mode.startswith("block"):       # unsplit: the prefill kernel's
+        assert lib.qwn_choose_gemm_splits(M // 16, T // 8, K // 32) == 1
     codes, scales = wl.random_packed_weight(M, K, seed=M + K + T, ksh=ksh)
     w = pkg.PackedWeight(codes, scales, M, K, k64=bool(ksh))
     x = wl.activations_normal(T, K, seed=T, outlier_frac=0.01)
@@ -48,20 +63,26 @@ def test_prefill_tile_widths(lib, pkg, orc, wl, mode, M, K, T, wrong_sums):
     # a result buffer whose rows start off 16 bytes in half of the cases
     off = 4 if wrong_sums else 0
     y = pkg.DevBuf(T * M * 4 + 16)
-    y.fill(0xA5)
+    at = np.ascontiguousarray(s.reshape(K // 32, T)[0]) if mode.startswith("token") else None
+    dat = _buf(pkg, at) if at is not None else None
     if mode == "w4a4":
-        assert lib.qwn_x_gemm_w4a4(w.ref, dq.ptr, ds.ptr, dsm.ptr, y.ptr + off, T) == 0
         rc, want = orc.gemm_w4a4(codes, scales, M, K, q, s, sm, T, fma=1)
-    elif mode.startswith("token"):
-        at = np.ascontiguousarray(s.reshape(K // 32, T)[0])
-        dat = _buf(pkg, at)
-        assert lib.qwn_x_gemm_w4a8_pertoken(w.ref, dq.ptr, dat.ptr, dsm.ptr, y.ptr + off, T, 0) == 0
+    elif at is not None:
         rc, want = orc.gemm_w4a8_pertoken(codes, scales, M, K, ksh, q, at, sm, T)
     else:
-        assert lib.qwn_x_gemm_w4a8(w.ref, dq.ptr, ds.ptr, dsm.ptr, y.ptr + off, T, None, 0) == 0
         rc, want = orc.gemm_w4a8(codes, scales, M, K, ksh, q, s, sm, T, fma=1)
-    lib.tq_sync()
-    assert rc == 0 and lib.tq_last_error() == 0
-    raw = y.to_numpy(np.uint8)
-    assert raw[off:off + T * M * 4].tobytes() == np.ascontiguousarray(want, dtype=np.float32).tobytes()
-    assert (raw[:off] == 0xA5).all() and (raw[off + T * M * 4:] == 0xA5).all()      # nothing beyond y
+    assert rc == 0
+    want = np.ascontiguousarray(want, dtype=np.float32).tobytes()
+    for _ in range(3):
+        y.fill(0xA5)
+        if mode == "w4a4":
+            assert lib.qwn_x_gemm_w4a4(w.ref, dq.ptr, ds.ptr, dsm.ptr, y.ptr + off, T) == 0
+        elif at is not None:
+            assert lib.qwn_x_gemm_w4a8_pertoken(w.ref, dq.ptr, dat.ptr, dsm.ptr, y.ptr + off, T, 0) == 0
+        else:
+            assert lib.qwn_x_gemm_w4a8(w.ref, dq.ptr, ds.ptr, dsm.ptr, y.ptr + off, T, None, 0) == 0
+        lib.tq_sync()
+        assert lib.tq_last_error() == 0
+        raw = y.to_numpy(np.uint8)
+        assert raw[off:off + T * M * 4].tobytes() == want
+        assert (raw[:off] == 0xA5).all() and (raw[off + T * M * 4:] == 0xA5).all()      # nothing beyond y
