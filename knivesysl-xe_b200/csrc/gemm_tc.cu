@@ -276,6 +276,8 @@ __device__ __forceinline__ void reg_dealloc() {
 
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&v)[16]) { tmem_ld16(taddr, v); }
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&v)[32]) { tmem_ld32(taddr, v); }
+__device__ __forceinline__ void tmem_wait_ldn(uint32_t (&v)[16]) { tmem_wait_ld16(v); }
+__device__ __forceinline__ void tmem_wait_ldn(uint32_t (&v)[32]) { tmem_wait_ld32(v); }
 
 // GW = k-tiles accumulated in TMEM before one fp32 promote (1: the reference's arithmetic with
 // a scale per (token, K32); 2: K64 weight groups with per-token activation scales, or - not
@@ -424,7 +426,7 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
 #pragma unroll
                 for (int c = 0; c < WT / kCols; ++c) {
                     tmem_ldn(lane_base + b * TN + c * kCols, d);
-                    tmem_wait_ld_all();
+                    tmem_wait_ldn(d);
                     if constexpr (kPacked) {
 #pragma unroll
                         for (int j = 0; j < kCols / 2; ++j)
