@@ -298,6 +298,10 @@ int qwn_dbg_tile_dots_gemv(const tq_qmma_weight_t *w, int32_t *d_out);
 int qwn_dbg_tile_dots_gemm(const tq_qmma_weight_t *w, const int8_t *d_aq, int T, int32_t *d_out);
 /* Copies of the prepared scratch (device->device), for tests: any pointer may be NULL. */
 int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum);
+/* 1 if the last tensor-core prefill call was done by the kernel variant for code sums that are
+ * not the sums of the codes (only where the weight has zero points), else 0; waits for the
+ * stream. -1: no such call yet. */
+int qwn_dbg_prefill_sums_variant(void);
 
 /* Model-free forms of the reference's self-checks and micro-benches
  * (xpu/src/kernels_dpas.cpp:2146-2333, 2613-2693): they take a weight record instead of

@@ -1117,4 +1117,6 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum) {
     return 0;
 }
 
+int qwn_dbg_prefill_sums_variant(void) { return tq::prefill_sums_variant(); }
+
 }  // extern "C"

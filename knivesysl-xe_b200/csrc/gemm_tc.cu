@@ -99,14 +99,31 @@ struct TcTile {
 // are 512 bytes apart; the second K = 16 instruction of a k-tile starts two chunks further
 constexpr uint32_t kLboH = 128, kSboH = 512;
 
+// Device words that say which variant of the GEMM does a call. The pre-pass stamps `diff` with the
+// generation if some asum of the call is not the sum of its codes, and `zp` if some zero point of the
+// weight is not 0; only where both are stamped does z * (sum of codes - asum) enter the result. The SUMS
+// kernel, last of the call, moves the generation on, so that nothing has to be cleared and a captured
+// call decides by the data of each replay.
+struct SumsState {
+    unsigned gen, diff, zp;      // read together, with `arrived`, as one 16-byte word
+    unsigned arrived;            // CTAs of the SUMS kernel that have read the words
+    unsigned last;               // the call before: did its SUMS kernel do the work?
+};
+// Stamps *word unless it is stamped already: a store by every CTA costs far more than the look (136
+// tokens on 10240 x 5120 with zero points: 167 us instead of 113, 258 with a store by every warp).
+__device__ __forceinline__ void stamp(unsigned *word, unsigned gen) {
+    if (__ldcg(word) != gen) *word = gen;
+}
+// Never 0, what the stamps start from.
+__device__ __forceinline__ unsigned next_generation(unsigned g) { return g + 1 ? g + 1 : 1; }
+
 struct TcParams {
     const uint8_t *wimg;     // per (128-row block, k-tile): kABytes of fp16 weights in operand layout
     const uint16_t *scales;
     const uint8_t *img;      // per (TN-token block, step): kImgStep bytes (see the pre-pass)
     void *y;
     const float *as_tok;     // per-token scales (PERTOK kernels)
-    const unsigned *sums_flag;   // == call: some asum of this call is not the sum of its codes
-    unsigned call;
+    SumsState *sums;
     int *status;
     unsigned long long wait_ns;   // limit of every mbarrier wait
     int M, Kt, ksh, T, tok_blocks, out_bf16;
@@ -155,8 +172,7 @@ struct PrepassArgs {
     const float *as;
     const int32_t *asum;
     uint8_t *wimg, *img;
-    unsigned *sums_flag;
-    unsigned call;
+    SumsState *sums;
     int M, Kt, ksh, T, TN, Tpad;
     int wblocks;             // CTAs that expand weights; the others convert activations
 };
@@ -172,21 +188,24 @@ struct PrepassArgs {
 //  * Activations: the caller's staging -> per (TN-token block, step of two k-tiles) the fp16
 //    codes of k-tile 0 then 1 as [TN / 8][4 K-chunks][8 tokens][16 B], as[2][TN], and
 //    (sum of the codes - asum)[2][TN], 0 unless the caller's asum is something else than the sum
-//    of its codes; in that case the flag selects the kernel that applies z times that difference.
+//    of its codes (SumsState).
 //    Tokens >= T are padded with zeros. S4: int4 codes; a K64 block's scale and sum go with its
 //    first k-tile.
 template <bool S4>
 __global__ void __launch_bounds__(256) gemm_tc_prepass_kernel(const PrepassArgs a) {
     pdl_trigger();
     pdl_wait();      // the images may still be read by the previous call's kernel
+    const unsigned gen = __ldcg(&a.sums->gen);
     if ((int)blockIdx.x < a.wblocks) {
         const uint32_t mask = 0x000F000Fu, bias = 0x64086408u;
         const size_t n = (size_t)a.M * a.Kt;
         const int Ktg = a.Kt >> a.ksh;
+        uint32_t any = 0;
         for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)a.wblocks * 256) {
             const int kt = (int)(i / a.M), m = (int)(i % a.M);
             const uint4 c4 = ldg_stream_v4(a.codes + ((size_t)(m >> 4) * a.Kt + kt) * 256 + (m & 15) * 16);
             const uint32_t sw = __ldg(a.scales + ((size_t)(m >> 4) * Ktg + (kt >> a.ksh)) * 16 + (m & 15));
+            any |= sw & 15u;
             const uint32_t base = (0x6400u + ((sw ^ 8u) & 15u)) * 0x00010001u;      // 1032 + z
             const int r = m & (kTM - 1);
             uint8_t *dst = a.wimg + ((size_t)(m / kTM) * a.Kt + kt) * kABytes + (r >> 3) * kSboH + (r & 7) * 16;
@@ -195,11 +214,13 @@ __global__ void __launch_bounds__(256) gemm_tc_prepass_kernel(const PrepassArgs 
             *reinterpret_cast<uint4 *>(dst + 2 * kLboH) = nib8_to_h8(c4.z, mask, bias, base);     // k 16..23
             *reinterpret_cast<uint4 *>(dst + 3 * kLboH) = nib8_to_h8(c4.w, mask, bias, base);     // k 24..31
         }
+        if (__syncthreads_or((int)any) && threadIdx.x == 0) stamp(&a.sums->zp, gen);
         return;
     }
     const int T = a.T, TN = a.TN, nsteps = a.Kt >> 1;
     const size_t nrow = (size_t)nsteps * a.Tpad;
     const size_t img_step = (size_t)TN * 144;
+    int diff = 0;
     for (size_t i = (size_t)(blockIdx.x - a.wblocks) * 256 + threadIdx.x; i < nrow;
          i += (size_t)(gridDim.x - a.wblocks) * 256) {
         const int st = (int)(i / a.Tpad), tok = (int)(i % a.Tpad);
@@ -259,8 +280,9 @@ __global__ void __launch_bounds__(256) gemm_tc_prepass_kernel(const PrepassArgs 
         sv[TN + tl] = s1;
         sv[2 * TN + tl] = (float)d0;
         sv[3 * TN + tl] = (float)d1;
-        if (d0 | d1) *a.sums_flag = a.call;
+        diff |= d0 | d1;
     }
+    if (__syncthreads_or(diff) && threadIdx.x == 0) stamp(&a.sums->diff, gen);
 }
 
 constexpr int kWaitMma = 21, kWaitEpi = 22, kWaitProd = 23;   // status codes of failed waits
@@ -289,8 +311,8 @@ __device__ __forceinline__ void tmem_wait_ldn(uint32_t (&v)[32]) { tmem_wait_ld3
 // n % NBP. A worker warp owns 32 TMEM lanes (rows) and WT of the tile's tokens.
 //
 // SUMS: the kernel applies z * (sum of codes - asum), for callers whose asum is not the sum of
-// their codes. Both variants are launched; the one the pre-pass's flag does not select returns
-// at once.
+// their codes, on weights with zero points. Both variants are launched; the one that SumsState does
+// not select returns at once.
 template <int GW, bool PERTOK, bool SUMS, int WT>
 __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
     using G = TcTile<WT>;
@@ -315,8 +337,16 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
     // fma on token pairs (5 % faster there; in every other mode the packed form measured slower).
     constexpr bool kPacked = PERTOK && !SUMS && GW == 2;
     pdl_trigger();
-    pdl_wait();      // everything below reads what earlier kernels wrote (flag, images)
-    if ((*p.sums_flag == p.call) != SUMS) return;
+    pdl_wait();      // everything below reads what earlier kernels wrote (words, images)
+    const uint4 sw = __ldcg(reinterpret_cast<const uint4 *>(p.sums));      // gen, diff, zp, arrived
+    if ((sw.y == sw.x && sw.z == sw.x) != SUMS) {
+        // A CTA that reads the words after this store finds old stamps: not selected either.
+        if (SUMS && blockIdx.x == 0 && threadIdx.x == 0) {
+            p.sums->last = 0;
+            p.sums->gen = next_generation(sw.x);
+        }
+        return;
+    }
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t bars[2 * kSS + 2 * NB];   // full[kSS], empty[kSS], accfull[NB], accempty[NB]
     __shared__ uint32_t tmem_base_s;
@@ -349,6 +379,11 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
+    // all threads of this CTA have read the words; the last CTA to say so moves the generation on
+    if (SUMS && threadIdx.x == 0 && atomicInc(&p.sums->arrived, gridDim.x - 1) == gridDim.x - 1) {
+        p.sums->last = 1;
+        p.sums->gen = next_generation(sw.x);
+    }
 
     const int spt = p.Kt >> 1;                           // steps per tile
     const int ntiles = (p.M / kTM) * p.tok_blocks;
@@ -615,8 +650,7 @@ struct TcScratch {
     size_t img_bytes = 0;
     uint8_t *wimg = nullptr;      // fp16 image of the call's weight (4 bytes per packed byte)
     size_t wimg_bytes = 0;
-    unsigned *sums_flag = nullptr;
-    unsigned calls = 0;
+    SumsState *sums = nullptr;
 } g_tc;
 
 int g_tc_sms = 0;
@@ -676,8 +710,9 @@ int launch_gemm_tc(const GemmTcArgs &a) {
         TQ_CHECK(cudaGetDevice(&dev));
         TQ_CHECK(cudaDeviceGetAttribute(&g_tc_sms, cudaDevAttrMultiProcessorCount, dev));
         if (g_tc_sms <= 0) g_tc_sms = 148;
-        g_tc.sums_flag = static_cast<unsigned *>(tq_dev_alloc(sizeof(unsigned), "gemm.tc.sums.flag"));
-        TQ_CHECK(cudaMemsetAsync(g_tc.sums_flag, 0, sizeof(unsigned), stream()));
+        g_tc.sums = static_cast<SumsState *>(tq_dev_alloc(sizeof(SumsState), "gemm.tc.sums.state"));
+        const SumsState first = {1, 0, 0, 0, 0};
+        TQ_CHECK(cudaMemcpyAsync(g_tc.sums, &first, sizeof first, cudaMemcpyHostToDevice, stream()));
     }
     ProfScope prof(a.M, a.K, a.T, a.aq4 ? 44 : (a.ksh ? 64 : 4));
     const int TN = choose_tile_tokens(a.M, a.T, g_tc_sms);
@@ -694,11 +729,10 @@ int launch_gemm_tc(const GemmTcArgs &a) {
         g_tc.wimg = static_cast<uint8_t *>(tq_dev_alloc(wbytes, "gemm.tc.weight.image"));
         g_tc.wimg_bytes = wbytes;
     }
-    if (++g_tc.calls == 0) ++g_tc.calls;        // never the flag's initial value
     PrepassArgs q{};
     q.codes = a.codes; q.scales = a.scales; q.as = a.as; q.asum = a.asum;
     q.aq = a.aq4 ? reinterpret_cast<const int8_t *>(a.aq4) : a.aq;
-    q.wimg = g_tc.wimg; q.img = g_tc.img; q.sums_flag = g_tc.sums_flag; q.call = g_tc.calls;
+    q.wimg = g_tc.wimg; q.img = g_tc.img; q.sums = g_tc.sums;
     q.M = a.M; q.Kt = Kt; q.ksh = a.ksh; q.T = a.T; q.TN = TN; q.Tpad = Tpad;
     // one round of CTAs (8 per SM), shared between the two jobs by their items
     const size_t witems = (size_t)a.M * Kt, aitems = (size_t)(Kt / 2) * Tpad * 3;
@@ -712,7 +746,7 @@ int launch_gemm_tc(const GemmTcArgs &a) {
     TcParams p{};
     p.wimg = g_tc.wimg; p.scales = a.scales; p.img = g_tc.img; p.y = a.y;
     p.as_tok = a.as_tok;
-    p.sums_flag = g_tc.sums_flag; p.call = g_tc.calls;
+    p.sums = g_tc.sums;
     p.status = device_status_word();
     p.wait_ns = wait_limit_ns();
     p.M = a.M; p.Kt = Kt; p.ksh = a.ksh; p.T = a.T; p.tok_blocks = tok_blocks; p.out_bf16 = a.out_bf16;
@@ -724,6 +758,15 @@ int launch_gemm_tc(const GemmTcArgs &a) {
     }
     TQ_LAUNCH_CHECK("gemm_w4a8_tc_kernel");
     return 0;
+}
+
+int prefill_sums_variant() {
+    if (!g_tc.sums) return -1;
+    unsigned last = 0;
+    if (cudaMemcpyAsync(&last, &g_tc.sums->last, sizeof last, cudaMemcpyDeviceToHost, stream()) != cudaSuccess ||
+        cudaStreamSynchronize(stream()) != cudaSuccess)
+        return -1;
+    return (int)last;
 }
 
 }  // namespace tq
