@@ -983,7 +983,7 @@ int window_groups(const GemmArgs &a) {
 // The ring kernel takes T = 8 calls whose split activations fit beside the rings.
 // Launch shape of the ring kernel for a call, or false when the call is not its to take.
 struct RingPlan {
-    int grid, nw, ns, nwin, ntg;
+    int grid, nw, ns, nwin, ntg, rounds;      // rounds: tasks that the busiest warp does one after the other
     size_t smem;
 };
 // Plan with `ntg` token groups per warp (token windows of 8 ntg tokens on CTA columns).
@@ -1015,18 +1015,27 @@ bool ring_plan_ntg(const GemmArgs &a, int ntg, RingPlan &p) {
         p.ns = 4;
         while (p.ns > 2 && (size_t)p.nw * p.ns * kRStage + fixed > kSmemLimit) --p.ns;
     }
+    p.rounds = (per_cta + p.nw - 1) / p.nw;
     p.smem = (size_t)p.nw * p.ns * kRStage + fixed;
     return p.smem <= kSmemLimit;
 }
-// The widest plan that fits: all of a call's tokens on one warp (weights and their unpacking
-// paid once), else windows of 32, 16 or 8 tokens on CTA columns. In per-token mode every number of
-// token groups has an instantiation; before 3, 5, 6 and 7 had one, 24 tokens ran as three windows
-// and 40 as five, each unpacking all weights (5120 x 17408 K32, us with staging: 24 tokens 43.5 -> 32.8,
-// 40: 122 -> 50, 48: 71 -> 58, 56: 125 -> 65). Two exceptions keep the windows: the reference's
-// arithmetic, whose split rule leaves few tasks per call (24 tokens 42.0 against 43.8 us on that
-// shape, 48 tokens 19.6 against 24.7 on 2 x 1024 x 5120), and 48 tokens whose splits are shorter than
-// four k-tiles, where the ordered reduction of the wider partials outweighs the unpacking
-// (3 x 1040 x 1088: 27.0 against 30.3 us).
+// Time of a plan's tasks, for choosing between two: the rounds that the busiest SM makes, each 5 for its
+// start and 3 for every token group of a task (tiles, staged activations, partials and their
+// reduction), up to twice as much where 21 to 32 warps share the SM instead of 20.
+int ring_cost(const RingPlan &p) { return p.rounds * (5 + 3 * p.ntg) * std::max(12, p.nw - 8); }
+
+// The widest power of two of token groups that divides the call's and fits: all tokens on one warp
+// (weights and their unpacking paid once), else windows of 32, 16 or 8 tokens on CTA columns. In
+// per-token mode 3, 5, 6 and 7 groups have instantiations too, so that 24, 40, 48 and 56 tokens need
+// not run as windows of 8 or 16 that each unpack all weights (5120 x 17408 K32, us with staging, windows
+// against one warp: 43.0 / 32.4, 120 / 49.7, 70.7 / 56.8, 124 / 64.8). With few row groups it is the other
+// way round: windows spread a call over more SMs, and the reduction of a split's wider partials is a
+// longer chain (512 x 1024: 8.3 / 12.4, 13.5 / 16.3, 11.4 / 17.5, 13.7 / 19.8). ring_cost() decides;
+// over 88 weights of 256 to 17408 rows (one to three of them), K 1024 to 17408, both scale groups
+// and these four token counts its choice is on average 0.1 % behind the faster plan; the largest
+// loss against windows is 7 % (1024 x 5120, 56 tokens: 23.7 / 25.3), against one warp none.
+// The reference's arithmetic keeps the powers of two: its split rule leaves few tasks per call
+// (24 tokens 42.0 against 43.8 us on 5120 x 17408, 48 tokens 19.6 against 24.7 on 2 x 1024 x 5120).
 bool ring_plan(const GemmArgs &a, RingPlan &p) {
     if (a.T < 8 || a.T > 64 || (a.T % 8) || a.dump) return false;
     if (a.x && (a.T != 8 || a.mode)) return false;   // the fused quantiser serves one window
@@ -1037,14 +1046,19 @@ bool ring_plan(const GemmArgs &a, RingPlan &p) {
         if (g_num_sms <= 0) g_num_sms = 148;
     }
     const int tg = a.T / 8;
-    const bool short_splits = (a.K >> 5) < 4 * a.max_splits;
-    auto has_kernel = [&](int ntg) {
-        if (!(ntg & (ntg - 1))) return true;                 // 8, 4, 2, 1
-        return a.mode && !(ntg == 6 && short_splits);
-    };
-    for (int ntg = 8; ntg >= 1; --ntg)
-        if (tg % ntg == 0 && has_kernel(ntg) && (ntg == 1 || !a.npeer) && ring_plan_ntg(a, ntg, p)) return true;
-    return false;
+    bool found = false;
+    for (int ntg = 8; ntg >= 1 && !found; ntg >>= 1)
+        found = tg % ntg == 0 && (ntg == 1 || !a.npeer) && ring_plan_ntg(a, ntg, p);
+    if (a.mode && !a.npeer)
+        for (int ntg = 7; ntg >= 3; --ntg) {
+            RingPlan wide;
+            if (tg % ntg || ntg == 4 || !ring_plan_ntg(a, ntg, wide)) continue;
+            if (!found || ring_cost(wide) < ring_cost(p)) {
+                p = wide;
+                found = true;
+            }
+        }
+    return found;
 }
 
 bool launch_ring(const GemmArgs &a) {

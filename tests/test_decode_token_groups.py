@@ -1,6 +1,6 @@
 """Per-token decode batches of 3, 5, 6 and 7 eight-token groups: all of a call's tokens on one warp
-(gemm_w4a8_ring_kernel), and the shapes around the rule that keeps 48 tokens with short splits in
-windows. Bit-identical to the oracle: integer dots, then the same fp32 operations in the same order."""
+(gemm_w4a8_ring_kernel) where a call has many row groups, windows of tokens on CTA columns where it
+has few. Bit-identical to the oracle: integer dots, then the same fp32 operations in the same order."""
 import numpy as np
 import pytest
 
@@ -10,10 +10,12 @@ import pytest
 @pytest.mark.parametrize("Ms,K,ksh", [
     ([5120], 1088, 0),          # many row groups: more tasks than warps
     ([5120], 1088, 1),
-    ([1040, 1040, 1040], 1088, 0),   # 16 splits of 2 or 3 k-tiles: 48 tokens stay in windows
-    ([16], 64, 1),              # one row group, one K64 group
-    ([272], 2112, 0),           # 4 k-tiles a split: the other side of that rule
-    ([48, 16], 4160, 1),        # splits of unequal length
+    ([1040, 1040, 1040], 1088, 0),   # 16 splits of 2 or 3 k-tiles; 48 tokens in windows of 24
+    ([16], 64, 1),              # one row group, one K64 group: windows of 8 or 16
+    ([272], 2112, 0),           # windows, 4 or 5 k-tiles a split
+    ([48, 16], 4160, 1),        # windows, splits of unequal length
+    ([2064, 48], 4160, 1),      # one warp, splits of unequal length
+    ([40976], 64, 1),           # one warp, one K64 group
 ])
 def test_pertoken_token_groups(lib, pkg, orc, wl, Ms, K, ksh, T):
     host = [wl.random_packed_weight(M, K, seed=M + K + T + i, ksh=ksh) for i, M in enumerate(Ms)]
