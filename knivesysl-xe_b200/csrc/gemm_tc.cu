@@ -498,15 +498,29 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
                         }
                     }
                 }
+                // Tell the MMA that it may overwrite the buffer and, behind the step's last group, the copy
+                // thread that the slot's images may be replaced. The copies write through the
+                // async proxy, which an arrive does not order behind this warp's shared-memory reads: in
+                // a kernel of 64-token tiles, whose workers take eight slots in a row at the start of a tile,
+                // reads still under way got the scales of the slot's next use (step n + 8; W4A4, a third of
+                // the calls). So the proxy fence comes first. With one group per step both arrives follow it
+                // as one instruction; with two, the accumulator is given back before it (4096 tokens:
+                // 1585 us against 1618 with the fence first and 1607 without; W4A4, 1024 tokens: 324
+                // against 318 and 318).
+                constexpr bool kOneArrive = kReadsSlot && GW == 2;
+                if (kOneArrive) fence_proxy_async_smem();
                 tc_fence_before();
                 __syncwarp();
-                // one instruction, two barriers: lane 0 tells the MMA that it may overwrite the
-                // buffer, lane 1 (behind the step's last group) the copy thread that the slot's
-                // images may be replaced
-                if (!kSlotFreedByMma && (GW == 2 || g == 1))
+                if (kOneArrive) {
                     mbar_arrive_if(lane == 0 ? accempty0 + b * 8 : empty0 + ss * 8, lane < 2);
-                else
+                } else {
                     mbar_arrive_if(accempty0 + b * 8, lane == 0);
+                    if (kReadsSlot && g == 1) {
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        mbar_arrive_if(empty0 + ss * 8, lane == 0);
+                    }
+                }
                 if (++b == NB) {
                     b = 0;
                     par ^= 1u;
@@ -679,9 +693,7 @@ void launch_mode(const GemmTcArgs &a, const TcParams &p, int grid) {
 // costs about (tokens + 96) units whatever the mode: on 10240 x 5120, K32 block scales, 136 tokens
 // took 66 / 80 / 100 us a round at 128 / 192 / 256 tokens a tile, and on 5120 x 17408
 // 224 / 270 / 345 us; the rest is how many rounds the tiles of that width need (136 tokens on the
-// first: 2 / 1 / 1 rounds, so 192). 64 tokens a tile (as many accumulator buffers as step slots) would
-// save short calls on few row blocks up to a quarter, but gave wrong words in W4A4 mode in up to half of
-// the runs for a reason not found, so that width does not exist; the others: none in 1500 runs each.
+// first: 2 / 1 / 1 rounds, so 192).
 int choose_tile_tokens(int M, int T, int sms) {
     int best = 0;
     long best_cost = 0;

@@ -9,6 +9,9 @@ twice, with odd step counts, within one tile and from tile to tile. Zero points 
 z * asum enters as z * sum(codes); an asum that is something else takes a kernel of its own. Every
 output word is compared with the oracle, which reads asum as given: all terms up to the promote are
 integers below 2^24 in either association, so no tolerance is needed."""
+import os
+import re
+
 import numpy as np
 import pytest
 
@@ -38,6 +41,21 @@ CASES = [(m, s) for m in MODES for s in SIZES + ONE_ROW_BLOCK["block" if m.start
 
 def _buf(pkg, a):
     return pkg.DevBuf.from_numpy(np.ascontiguousarray(a))
+
+
+def test_slots_are_released_behind_a_proxy_fence():
+    """The next bulk copy into a slot writes through the async proxy, so the workers' reads of it are
+    fenced before the arrive that allows it (read from the source: a copy that comes too early shows
+    only in the timing of some runs)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    with open(os.path.join(root, "knivesysl-xe_b200", "csrc", "gemm_tc.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    workers = text[text.index("if (warp < kWorkWarps)"):text.index("reg_dealloc<kRoleRegs>();")]
+    releases = [m.start() for m in re.finditer(r"mbar_arrive_if\([^;]*empty0 \+ ss", workers)]
+    assert releases
+    for at in releases:
+        last_read = max(workers.rfind("= sv[", 0, at), workers.rfind("sv_base +", 0, at))
+        assert "fence_proxy_async_smem();" in workers[last_read:at]
 
 
 @pytest.mark.gpu
