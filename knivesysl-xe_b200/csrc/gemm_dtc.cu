@@ -186,7 +186,7 @@ __global__ void __launch_bounds__(Cfg<TN>::kThreads, 1) gemm_w4a8_dtc_kernel(con
     if (threadIdx.x == 0) {
         for (int s = 0; s < kSlots; ++s) {
             mbar_init(full0 + s * 8, 4);         // one arrive per producer warp
-            mbar_init(accfull0 + s * 8, 1);      // tcgen05.commit
+            mbar_init(accfull0 + s * 8, 2);      // tcgen05.commit; the committing thread (below)
             mbar_init(empty0 + s * 8, EW);       // one arrive per epilogue warp
         }
         dead_s = 0;
@@ -572,6 +572,9 @@ __global__ void __launch_bounds__(Cfg<TN>::kThreads, 1) gemm_w4a8_dtc_kernel(con
                     }
                     DTC_STAMP(2, 7)
                     tc_commit(accfull0 + slot * 8);
+                    // a commit tracks MMAs only; this arrival passes on that the slot is filled to the
+                    // epilogue warps, which read scales from it behind this barrier
+                    mbar_arrive(accfull0 + slot * 8);
                 }
                 DTC_STAMP(2, 1)
                 __syncwarp();
