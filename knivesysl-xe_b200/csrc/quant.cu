@@ -925,13 +925,21 @@ void launch_quant_chunk_s4(const float *d_x, int K, int T, uint8_t *d_aq4, float
     TQ_LAUNCH_CHECK("quant_chunk_s4_kernel");
 }
 
+// Rows and codes that take 16-byte loads and 4-byte stores (K is a multiple of 32, so the start decides).
+static bool vector_rows(const void *rows, const int8_t *d_aq) {
+    return (reinterpret_cast<uintptr_t>(rows) & 15) == 0 && (reinterpret_cast<uintptr_t>(d_aq) & 3) == 0;
+}
+
 // Decode batches: a cluster of 8, 4 or 2 CTAs per token when the row divides into K32-aligned
-// slices of at most 4096 values. False: the shape is not covered, nothing was launched.
+// slices of at most 4096 values and the buffers take its vector accesses. False: the call is not
+// covered, nothing was launched.
 constexpr int kClusterMaxT = 64;     // above, the per-token and wide kernels measured faster
 template <int SRC>
 bool launch_quant_cluster(const ClusterSrc &src, int K, int T, int8_t *d_aq, float *d_as, int32_t *d_asum,
                           float *d_as_tok, const SyncArgs &sa) {
-    if (T > kClusterMaxT) return false;
+    if (T > kClusterMaxT || !vector_rows(src.x, d_aq) || !vector_rows(src.x2, d_aq) || !vector_rows(src.out, d_aq) ||
+        (reinterpret_cast<uintptr_t>(src.w) & 7))
+        return false;
     for (unsigned c = 8; c >= 2; c >>= 1) {
         if (K % (32 * (int)c) || K / (int)c > 4096) continue;
         launch_pdl_cluster(quant_chunk_pertoken_cluster_kernel<SRC>, dim3(c, T), dim3(256), c, src, K, T, d_aq,
@@ -969,19 +977,20 @@ void launch_quant_chunk_pertoken(const float *d_x, int K, int T, int8_t *d_aq, f
     if (launch_quant_cluster<0>(ClusterSrc{d_x, nullptr, nullptr, nullptr, 0.0f}, K, T, d_aq, d_as, d_asum,
                                 d_as_tok, sa))
         return;
-    if (T <= 32 && K <= 8192) {
+    const bool vec = vector_rows(d_x, d_aq);
+    if (vec && T <= 32 && K <= 8192) {
         launch_pdl(quant_chunk_pertoken_regs_kernel<1024, 2>, dim3(T), dim3(1024), 0, d_x, K, T, d_aq, d_as,
                    d_asum, d_as_tok, sa);
         TQ_LAUNCH_CHECK("quant_chunk_pertoken_regs_kernel");
         return;
     }
-    if (T <= 32) {
+    if (vec && T <= 32) {
         launch_pdl(quant_chunk_pertoken_fused_kernel, dim3(T), dim3(1024), 0, d_x, K, T, d_aq, d_as,
                    d_asum, d_as_tok, sa);
         TQ_LAUNCH_CHECK("quant_chunk_pertoken_fused_kernel");
         return;
     }
-    if (K <= 8192 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0 && (reinterpret_cast<uintptr_t>(d_aq) & 3) == 0) {
+    if (vec && K <= 8192) {
         // a row fits the registers of one CTA: one pass whatever the token count
         launch_pdl(quant_chunk_pertoken_regs_kernel<256, 8>, dim3(T), dim3(256), 0, d_x, K, T, d_aq, d_as,
                    d_asum, d_as_tok, sa);
