@@ -84,17 +84,12 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // loop with its clock arithmetic at each of them multiplies the kernel's code size until its
 // roles evict one another from the instruction cache.
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, int *status, int code,
-                                                   uint64_t limit_ns, uint32_t suspend_ns = 0) {
-    // mbarrier.try_wait comes back after some tens of clocks while the phase is incomplete, so
-    // a warp that polls back to back takes a fifth or more of its scheduler's issue slots
-    // from the warps beside it. A single issuing thread that waits beside working warps
-    // passes suspend_ns > 0: the wait then carries that suspend-time hint and the thread
-    // stays off the scheduler until the phase completes or the time is up (measured a little
-    // faster than a nanosleep between polls, which wakes late). The clock is read every 2048
-    // polls, so the limit is noticed within 2048 * suspend_ns.
+                                                   uint64_t limit_ns) {
+    // The clock is read every 2048 polls; mbarrier.try_wait comes back after some tens of clocks
+    // while the phase is incomplete.
     uint64_t t0 = 0;
     for (uint32_t polls = 1;; ++polls) {
-        if (suspend_ns ? mbar_try_wait_hint(bar, parity, suspend_ns) : mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if ((polls & 2047u) == 0) {
             const uint64_t now = global_timer_ns();
             if (t0 == 0) t0 = now;
