@@ -40,7 +40,7 @@
 // 50 / 41 % busy and the tensor pipe 23 / 55 %. With two 256-column buffers a group's cycle is MMA,
 // hand-off, promote, hand-off, overlapped with one other group. Measured, staging included, against
 // 128-token tiles with the zero point applied in the promote: 17408 x 5120 K64, 4096 tokens in the
-// reference's arithmetic 1.60 against 1.77 ms; 2048 tokens with per-token scales 0.43 against
+// reference's arithmetic 1.59 against 1.77 ms; 2048 tokens with per-token scales 0.43 against
 // 0.49 ms; 1024 tokens W4A4 with zero points 0.32 against 0.57 ms; 5120 x 17408, 1000 tokens, zero
 // points 0.60 against 0.88 ms; 10240 x 5120 K32, 136 tokens, zero points 114 against 216 us.
 // Wider tiles pay a group's fixed work (barrier, scale word, counters: about 70 instructions) once
@@ -72,12 +72,16 @@ constexpr int kMmaWarps = 2;
 constexpr int kThreads = (kWorkWarps + 4) * 32;
 // A launch with 20 warps gives every thread 96 registers (61440 of the SM's); the workers of the
 // widest tile, whose 64 accumulators and loaded columns do not fit in that, take 104 and the other
-// four warps keep 64: 512 * 104 + 128 * 64 = 61440, exactly what the launch holds. (112 and 32:
-// the MMA and copy threads spill, and per-token prefill of 4096 tokens took 0.80 instead of 0.69 ms.)
+// four warps keep 64: 512 * 104 + 128 * 64 = 61440, exactly what the launch holds. A few words still
+// spill at that split: 8 bytes a thread in block mode and 12 (40 loaded) in W4A4 at 256 tokens, none
+// with per-token scales, up to 88 in the SUMS variants. (112 and 32: the MMA and copy threads spill
+// too, and per-token prefill of 4096 tokens took 0.80 instead of 0.69 ms.)
 constexpr int kLaunchRegs = 96, kWorkRegs = 104, kRoleRegs = 64;
 static_assert(kWorkWarps * 32 * kWorkRegs + 4 * 32 * kRoleRegs <= kThreads * kLaunchRegs,
               "the register split must not exceed what the launch holds");
-constexpr uint32_t kNapNs = 2000;        // suspend-time hint of the waits
+// Suspend-time hint of the waits: a thread that polls back to back takes issue slots from the warps
+// beside it, one that waits with the hint stays off the scheduler until the phase completes.
+constexpr uint32_t kNapNs = 2000;
 
 // Geometry of a tile of TN = 4 * WT tokens (a worker thread promotes WT of them).
 template <int WT>
@@ -689,11 +693,14 @@ void launch_mode(const GemmTcArgs &a, const TcParams &p, int grid) {
     else launch_both<1, true, WT>(p, grid);
 }
 
-// Tokens per tile: the width whose rounds of tiles over the SMs cost least. A round of tiles
-// costs about (tokens + 96) units whatever the mode: on 10240 x 5120, K32 block scales, 136 tokens
-// took 66 / 80 / 100 us a round at 128 / 192 / 256 tokens a tile, and on 5120 x 17408
-// 224 / 270 / 345 us; the rest is how many rounds the tiles of that width need (136 tokens on the
-// first: 2 / 1 / 1 rounds, so 192).
+// Tokens per tile: the width whose rounds of tiles over the SMs cost least, a round counted as
+// (tokens + 96) units. One constant for five modes whose own ones differ: a round of 148 tiles takes,
+// at 128 / 192 / 256 tokens and K 5120, 63 / 78 / 102 us in block mode on K32 weights (constant 83),
+// 58 / 78 / 102 on K64 (45), 48 / 56 / 69 with per-token scales on K32 (172; 89 at K 2048),
+// 25 / 35 / 42 on K64 (57), 39 / 51 / 66 in W4A4 (56). The rest is how many rounds the tiles of a width
+// need (136 tokens on 10240 rows: 2 / 1 / 1 rounds, so 192). Over 128 to 2048 tokens on 10240 x 5120,
+// 5120 x 17408, 17408 x 5120 and 2048 x 5120 in these modes the choice is at most 3.5 % behind the
+// fastest width (17408 x 5120, K64 blocks, 776 tokens: 453 us at 256, 438 at 192).
 int choose_tile_tokens(int M, int T, int sms) {
     int best = 0;
     long best_cost = 0;
