@@ -1028,7 +1028,7 @@ int ring_cost(const RingPlan &p) { return p.rounds * (5 + 3 * p.ntg) * std::max(
 // (weights and their unpacking paid once), else windows of 32, 16 or 8 tokens on CTA columns. In
 // per-token mode 3, 5, 6 and 7 groups have instantiations too, so that 24, 40, 48 and 56 tokens need
 // not run as windows of 8 or 16 that each unpack all weights (5120 x 17408 K32, us with staging, windows
-// against one warp: 43.0 / 32.4, 120 / 49.7, 70.7 / 56.8, 124 / 64.8). With few row groups it is the other
+// against one warp: 42.7 / 32.2, 120 / 49.7, 70.7 / 56.8, 124 / 64.8). With few row groups it is the other
 // way round: windows spread a call over more SMs, and the reduction of a split's wider partials is a
 // longer chain (512 x 1024: 8.3 / 12.4, 13.5 / 16.3, 11.4 / 17.5, 13.7 / 19.8). ring_cost() decides;
 // over 88 weights of 256 to 17408 rows (one to three of them), K 1024 to 17408, both scale groups
