@@ -71,6 +71,20 @@ __device__ __forceinline__ uint32_t mbar_test_wait(uint32_t bar, uint32_t parity
     return ok;
 }
 
+// The same by a whole converged warp: true if every lane finds the phase complete, in all lanes.
+__device__ __forceinline__ bool mbar_test_wait_warp(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "vote.sync.all.pred q, p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
 // Bounded wait: polls until the phase completes or limit_ns of wall clock have passed
 // (%globaltimer; the host passes tq::wait_limit_ns(), two seconds unless
 // tq_set_wait_limit_ms changed it), then records `code` in *status (first failure wins) and

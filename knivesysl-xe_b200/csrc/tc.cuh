@@ -57,15 +57,15 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
         : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], M = 128, K = 16 fp16 elements, fp32 accumulate. On operands
+// D[tmem] (+)= A[smem] * B[smem], M = 128, K = 32 e4m3 elements, fp32 accumulate. On operands
 // that hold small integers (products and sums below 2^24) the accumulator is the exact
 // integer dot: the tensor core adds fp32-exactly in that range.
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                           uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
+                                          uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
         :
         : "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
@@ -100,6 +100,12 @@ __device__ __forceinline__ void tmem_st16_const(uint32_t taddr, uint32_t c) {
         "r"(c), "r"(c), "r"(c), "r"(c), "r"(c)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr)
+                 : "memory");
+}
 // 8-column forms, and stores from a caller-held register array (kept live and distinct with
 // make_const_regs, so re-arming an accumulator costs the one store instruction).
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
@@ -113,6 +119,20 @@ __device__ __forceinline__ void tmem_wait_ld8(uint32_t (&v)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]),
                    "+r"(v[6]), "+r"(v[7])
+                 :
+                 : "memory");
+}
+// one wait for two loads
+__device__ __forceinline__ void tmem_wait_ld8x2(uint32_t (&v)[8], uint32_t (&w)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3]), "+r"(w[4]), "+r"(w[5]), "+r"(w[6]), "+r"(w[7])
+                 :
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld4x2(uint32_t (&v)[4], uint32_t (&w)[4]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(w[0]), "+r"(w[1]), "+r"(w[2]), "+r"(w[3])
                  :
                  : "memory");
 }
@@ -134,28 +154,7 @@ __device__ __forceinline__ void make_const_regs(uint32_t (&c)[N], uint32_t v) {
 #pragma unroll
     for (int i = 0; i < N; ++i) asm volatile("mov.b32 %0, %1;" : "=r"(c[i]) : "r"(v));
 }
-// 32-column forms (one instruction where four 16-column ones would each cost the issuing
-// thread on the order of a hundred clocks).
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                 : "r"(taddr)
-                 : "memory");
-}
-// The wait for a 32-column load; like tmem_wait_ld16 it ties the loaded registers, so that no use of
-// them, not even a copy, can come before it. (The prefill kernel with untied waits measures the same:
-// 614.7 against 614.3 us for 5120 x 17408, 1000 tokens; 1647 against 1646 for 17408 x 5120, 4096.)
-__device__ __forceinline__ void tmem_wait_ld32(uint32_t (&v)[32]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]),
-                   "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]),
-                   "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]),
-                   "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
-                 :
-                 : "memory");
-}
-// The same where the loaded values are not used any more (a kernel's teardown).
+// A wait for loads whose values are not used any more (a kernel's teardown).
 __device__ __forceinline__ void tmem_wait_ld_all() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -191,14 +190,8 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(kLbo >> 4) << 16) |
            ((uint64_t)(kSbo >> 4) << 32) | (1ull << 46);   // version 1, base offset 0, no swizzle
 }
-// The same layout with any chunk and row-group distances (16-bit operands: four 16-byte
-// K-chunks per row of a 32-element k-tile, so row groups are 512 bytes apart).
-__device__ __forceinline__ uint64_t smem_desc_at(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) |
-           ((uint64_t)(sbo >> 4) << 32) | (1ull << 46);
-}
-// instruction descriptor of kind::f16: D = f32 (1), A and B fp16 (0), both K-major
-__host__ __device__ constexpr uint32_t idesc_f16(int m, int n) {
+// instruction descriptor of kind::f8f6f4: D = f32 (1), A and B e4m3 (0), both K-major
+__host__ __device__ constexpr uint32_t idesc_f8(int m, int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 // instruction descriptor of kind::i8: D = s32 (2), A and B signed 8 bit (1), both K-major,
