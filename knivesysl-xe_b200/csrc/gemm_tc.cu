@@ -131,13 +131,13 @@ __host__ __device__ constexpr int image_step_bytes(bool int4) { return (int4 ? 6
 
 // Device words that say which variant of the GEMM does a call. The pre-pass stamps `diff` with the
 // generation if some asum of the call is not the sum of its codes, and `zp` if some zero point of the
-// weight is not 0; only where both are stamped does z * (sum of codes - asum) enter the result. The SUMS
-// kernel, last of the call, moves the generation on, so that nothing has to be cleared and a captured
+// weight is not 0; only where both are stamped does z * (sum of codes - asum) enter the result. The call's
+// last kernel moves the generation on, so that nothing has to be cleared and a captured
 // call decides by the data of each replay.
 struct SumsState {
     unsigned gen, diff, zp;      // read together, with `arrived`, as one 16-byte word
-    unsigned arrived;            // CTAs of the SUMS kernel that have read the words
-    unsigned last;               // the call before: did its SUMS kernel do the work?
+    unsigned arrived;            // CTAs of the last kernel that have read the words
+    unsigned last;               // the call before: did it apply the sums?
 };
 // Stamps *word unless it is stamped already: a store by every CTA costs far more than the look (136
 // tokens on 10240 x 5120 with zero points: 167 us instead of 113, 258 with a store by every warp).
@@ -365,11 +365,10 @@ __device__ __forceinline__ ulonglong2 lds_pairs(uint32_t addr) {
 // (counted across its tiles) uses step slot n % kSlots, promote group n uses accumulator buffer
 // n % NB. A worker warp owns 32 TMEM lanes (a row of each row block) and WT of the tile's tokens.
 //
-// SUMS: the kernel applies z * (sum of codes - asum), for callers whose asum is not the sum of
-// their codes, on weights with zero points. Both variants are launched; the one that SumsState does
-// not select returns at once.
-template <int MODE, bool SUMS, int WT>
-__global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
+// SUMS: z * (sum of codes - asum) is applied, for callers whose asum is not the sum of
+// their codes, on weights with zero points. ADVANCE: this is the call's last kernel.
+template <int MODE, bool SUMS, bool ADVANCE, int WT>
+__device__ __forceinline__ void tc_gemm(const TcParams &p, const unsigned gen) {
     using G = TcTile<MODE, WT>;
     constexpr int TN = G::TN, NB = G::NB, kSS = G::kSlots, R = G::R, GW = G::GW;
     constexpr bool PERTOK = G::kPerTok;
@@ -390,17 +389,6 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
     // The same for the slots: each is always filled for the same thread, or the accumulator that the
     // thread's previous step needed was free only after the slot's previous use had been promoted.
     static_assert(kByTile || kSS % kMmaWarps == 0 || kSS >= NB / (GW == 1 ? 2 : 1) + kMmaWarps, "slot phases");
-    pdl_trigger();
-    pdl_wait();      // everything below reads what earlier kernels wrote (words, images)
-    const uint4 sw = __ldcg(reinterpret_cast<const uint4 *>(p.sums));      // gen, diff, zp, arrived
-    if ((sw.y == sw.x && sw.z == sw.x) != SUMS) {
-        // A CTA that reads the words after this store finds old stamps: not selected either.
-        if (SUMS && blockIdx.x == 0 && threadIdx.x == 0) {
-            p.sums->last = 0;
-            p.sums->gen = next_generation(sw.x);
-        }
-        return;
-    }
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint64_t bars[2 * kSS + 2 * NB];   // full[kSS], empty[kSS], accfull[NB], accempty[NB]
     __shared__ uint32_t tmem_base_s;
@@ -434,9 +422,9 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
     tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
     // all threads of this CTA have read the words; the last CTA to say so moves the generation on
-    if (SUMS && threadIdx.x == 0 && atomicInc(&p.sums->arrived, gridDim.x - 1) == gridDim.x - 1) {
-        p.sums->last = 1;
-        p.sums->gen = next_generation(sw.x);
+    if (ADVANCE && threadIdx.x == 0 && atomicInc(&p.sums->arrived, gridDim.x - 1) == gridDim.x - 1) {
+        p.sums->last = SUMS;
+        p.sums->gen = next_generation(gen);
     }
 
     const int spt = p.Kt >> 1;                           // steps per tile
@@ -768,6 +756,35 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
     asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
 }
 
+// The call's data decide between the two forms (SumsState). A kernel of a narrow tile holds both behind one
+// branch: the second launch, which returns at once, takes about 2 us of every call (10240 x 5120, 136 tokens: 69.9 us
+// with it, 67.8 without; 1024 x 1024: 17.6 and 15.5). With more than kOneKernel accumulators a thread the
+// registers of one form spill for the other's sake (17408 x 5120, 4096 tokens, 64 accumulators: 1687 against
+// 1450 us), so there each is a kernel, both are launched and the one not selected returns.
+constexpr int kOneKernel = 40;
+enum Form { kPlain, kSums, kBothForms };
+template <int MODE, int WT, int FORM>
+__global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
+    pdl_trigger();
+    pdl_wait();      // everything below reads what earlier kernels wrote (words, images)
+    const uint4 sw = __ldcg(reinterpret_cast<const uint4 *>(p.sums));      // gen, diff, zp, arrived
+    const bool sums = sw.y == sw.x && sw.z == sw.x;
+    if (FORM == kBothForms ? sums : FORM == kSums) {
+        if (FORM == kSums && !sums) {
+            // A CTA that reads the words after this store finds old stamps: not selected either.
+            if (blockIdx.x == 0 && threadIdx.x == 0) {
+                p.sums->last = 0;
+                p.sums->gen = next_generation(sw.x);
+            }
+            return;
+        }
+        if constexpr (FORM != kPlain) tc_gemm<MODE, true, FORM != kPlain, WT>(p, sw.x);
+    } else {
+        if (FORM == kPlain && sums) return;
+        if constexpr (FORM != kSums) tc_gemm<MODE, false, FORM == kBothForms, WT>(p, sw.x);
+    }
+}
+
 struct TcScratch {
     uint8_t *img = nullptr;
     size_t img_bytes = 0;
@@ -779,36 +796,43 @@ struct TcScratch {
 int g_tc_sms = 0;
 
 template <int MODE, int WT>
-void launch_both(const TcParams &p, int sms) {
+void launch_tile(const TcParams &p, int sms) {
     using G = TcTile<MODE, WT>;
-    static bool once = false;
-    if (!once) {
-        for (auto k : {gemm_w4a8_tc_kernel<MODE, false, WT>, gemm_w4a8_tc_kernel<MODE, true, WT>})
-            TQ_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmem));
-        once = true;
-    }
     const int grid = std::min(sms, (p.M / kTM + G::R - 1) / G::R * p.tok_blocks);
-    launch_pdl(gemm_w4a8_tc_kernel<MODE, false, WT>, dim3(grid), dim3(kThreads), (size_t)G::kSmem, p);
-    launch_pdl(gemm_w4a8_tc_kernel<MODE, true, WT>, dim3(grid), dim3(kThreads), (size_t)G::kSmem, p);
+    auto go = [&](auto form) {
+        constexpr auto kernel = gemm_w4a8_tc_kernel<MODE, WT, decltype(form)::value>;
+        static bool once = false;
+        if (!once) {
+            TQ_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmem));
+            once = true;
+        }
+        launch_pdl(kernel, dim3(grid), dim3(kThreads), (size_t)G::kSmem, p);
+    };
+    if constexpr (G::R * WT <= kOneKernel) {
+        go(std::integral_constant<int, kBothForms>{});
+    } else {
+        go(std::integral_constant<int, kPlain>{});
+        go(std::integral_constant<int, kSums>{});
+    }
 }
 
 template <int MODE>
 void launch_width(const TcParams &p, int TN, int sms) {
     if constexpr (TcTile<MODE, 32>::R == 2) {
         switch (TN) {
-            case 128: launch_both<MODE, 32>(p, sms); break;
-            case 112: launch_both<MODE, 28>(p, sms); break;
-            case 96: launch_both<MODE, 24>(p, sms); break;
-            case 80: launch_both<MODE, 20>(p, sms); break;
-            case 64: launch_both<MODE, 16>(p, sms); break;
-            case 48: launch_both<MODE, 12>(p, sms); break;
-            default: launch_both<MODE, 8>(p, sms); break;
+            case 128: launch_tile<MODE, 32>(p, sms); break;
+            case 112: launch_tile<MODE, 28>(p, sms); break;
+            case 96: launch_tile<MODE, 24>(p, sms); break;
+            case 80: launch_tile<MODE, 20>(p, sms); break;
+            case 64: launch_tile<MODE, 16>(p, sms); break;
+            case 48: launch_tile<MODE, 12>(p, sms); break;
+            default: launch_tile<MODE, 8>(p, sms); break;
         }
     } else {
         switch (TN) {
-            case 256: launch_both<MODE, 64>(p, sms); break;
-            case 192: launch_both<MODE, 48>(p, sms); break;
-            default: launch_both<MODE, 32>(p, sms); break;
+            case 256: launch_tile<MODE, 64>(p, sms); break;
+            case 192: launch_tile<MODE, 48>(p, sms); break;
+            default: launch_tile<MODE, 32>(p, sms); break;
         }
     }
 }
