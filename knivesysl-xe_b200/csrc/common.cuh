@@ -438,6 +438,11 @@ __device__ __forceinline__ uint4 ldg_stream_v4(const void *p) {
                  : "l"(p));
     return v;
 }
+__device__ __forceinline__ uint2 ldg_stream_v2(const void *p) {
+    uint2 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ uint32_t ldg_stream_u32(const void *p) {
     uint32_t v;
     asm volatile("ld.global.nc.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(p));

@@ -8,9 +8,10 @@
 // mapping (a half-warp per tile, the two halves of a warp = the reference's two accumulators,
 // a team of S warps per row-group, partial sums added in split order through shared memory)
 // with plain batched loads: the one weight this tier serves in practice is hundreds of
-// megabytes, so ramp and tail do not matter. The GEMM gives a warp one (row-group, eight
+// megabytes, so ramp and tail do not matter. The general GEMM gives a warp one (row-group, eight
 // tokens) task, as the reference does, on mma.sync m16n8k32: its A fragment is word c and
-// word 4 + c of rows r and r + 8 of the tile, read straight from global memory.
+// word 4 + c of rows r and r + 8 of the tile, read straight from global memory. It is left for
+// activations that do not fit in shared memory (K above 25,800) and for unaligned buffers.
 #include "stream.cuh"
 
 #include <algorithm>
@@ -138,6 +139,128 @@ gemm_w8a8_kernel(const uint8_t *__restrict__ codes, const uint16_t *__restrict__
     }
 }
 
+// The same with the activations of a token window in shared memory: a warp takes a row-group and 8 NTG tokens.
+// What bounded the kernel above at 8 tokens was not the weight stream but its reads of the activations: every
+// warp of an SM comes to a k-tile's 256 bytes at about the same time and waits out an L2 latency for them. Here
+// one CTA per SM and window stages them once; a warp walks row-groups and keeps two register batches of U k-tiles
+// of its weight stream, the first one requested before the wait for the staging kernel. W = 28 warps
+// (72 registers) carry the 27.7 row-groups per SM of a 65536-row head in one round; with few row-groups
+// 16 warps with room for twice the tiles and no spills are faster (20000 x 2048, 8 tokens: 18.5 against 22.2 us
+// with 28; 65536 x 5120: 79.9 against 62.6). us of the whole call, kernel above / this one:
+// 65536 x 5120 at 8 / 16 / 32 tokens 69 / 113 / 226 -> 62 / 67 / 93; 20000 x 2048 22 / 26 / 45 -> 18 / 18 / 22;
+// 8192 x 5120 at 32 tokens 52 -> 41.
+constexpr int kSActTile = 256 + 32;        // staged codes and scales of a k-tile and eight tokens
+constexpr size_t kSSmem = 227 * 1024;
+constexpr int kWide = 28, kNarrow = 16;    // warps per CTA
+
+template <int NTG, int U, int W>
+__global__ void __launch_bounds__(W * 32, 1)
+gemm_w8a8_staged_kernel(const uint8_t *__restrict__ codes, const uint16_t *__restrict__ scales,
+                        const int8_t *__restrict__ aq, const float *__restrict__ as,
+                        float *__restrict__ y, int M, int Kt, int T) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int r = lane >> 2, c = lane & 3;
+    const int groups = M / 16, tok0 = blockIdx.y * (8 * NTG);
+    const int first = blockIdx.x + gridDim.x * warp, stride = gridDim.x * nw;
+    // Lane (r, c) holds k = 8c..8c+7 of rows r and r + 8 as the fragment's two k positions, and takes the
+    // same bytes of token r: a 32-byte row is one 8-byte load of four lanes.
+    const uint32_t lane_c = r * 32 + c * 8;
+    // one batch: the codes of U tiles, and their scales, two a lane
+    auto load = [&](uint2 (&w)[U][2], uint32_t &sc, int g, int kt0) {
+        const uint8_t *cp = codes + ((size_t)g * Kt + kt0) * 512u + lane_c;
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (kt0 + u < Kt) {
+                w[u][0] = ldg_stream_v2(cp + u * 512);
+                w[u][1] = ldg_stream_v2(cp + u * 512 + 256);
+            }
+        if ((lane >> 3) < U && kt0 + (lane >> 3) < Kt) sc = ldg_stream_u32(scales + ((size_t)g * Kt + kt0) * 16u + lane * 2);
+    };
+    uint2 w0[U][2], w1[U][2];
+    uint32_t s0 = 0, s1 = 0;
+    pdl_trigger();
+    if (first < groups) load(w0, s0, first, 0);
+    pdl_wait();      // so far only weights were read
+    const uint32_t act = smem_u32(smem);
+    for (int i = threadIdx.x; i < Kt * NTG * 16; i += blockDim.x) {       // 16 bytes of codes each
+        const int kt = i / (NTG * 16), rem = i - kt * (NTG * 16);
+        cp_async16_plain(act + (uint32_t)(kt * NTG + (rem >> 4)) * kSActTile + (rem & 15) * 16,
+                         aq + ((size_t)kt * T + tok0) * 32 + rem * 16);
+    }
+    for (int i = threadIdx.x; i < Kt * NTG * 8; i += blockDim.x) {        // one scale each
+        const int kt = i / (NTG * 8), rem = i - kt * (NTG * 8);
+        cp_async4(act + (uint32_t)(kt * NTG + (rem >> 3)) * kSActTile + 256 + (rem & 7) * 4,
+                  as + (size_t)kt * T + tok0 + rem);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    const f32x2 neg_magic = pack2(-kMagicF, -kMagicF);
+    int cmagic[4];
+    make_const_quad(cmagic, kMagicBits);
+    f32x2 acc01[NTG], acc23[NTG];
+    auto batch = [&](uint2 (&w)[U][2], uint32_t sc, int kt0) {
+        const uint32_t at = act + (uint32_t)(kt0 * NTG) * kSActTile;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (kt0 + u >= Kt) break;
+            const uint32_t sa = __shfl_sync(0xffffffffu, sc, u * 8 + (r >> 1));
+            const uint32_t sb = __shfl_sync(0xffffffffu, sc, u * 8 + 4 + (r >> 1));
+            const int sh = (r & 1) * 16;
+            const float ws0 = __half2float(__ushort_as_half((unsigned short)(sa >> sh)));
+            const float ws1 = __half2float(__ushort_as_half((unsigned short)(sb >> sh)));
+            const f32x2 ws0p = pack2(ws0, ws0), ws1p = pack2(ws1, ws1);
+#pragma unroll
+            for (int t = 0; t < NTG; ++t) {
+                uint2 b;
+                f32x2 as2;
+                const uint32_t tile = at + (u * NTG + t) * kSActTile;
+                asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(b.x), "=r"(b.y) : "r"(tile + lane_c));
+                asm volatile("ld.shared.u64 %0, [%1];" : "=l"(as2) : "r"(tile + 256 + c * 8));
+                int d[4];      // the dot + kMagicBits: as fp32, 12582912 + dot
+                mma_s8_c(d, w[u][0].x, w[u][1].x, w[u][0].y, w[u][1].y, b.x, b.y, cmagic);
+                fma2_acc(acc01[t], add2(pack2i(d[0], d[1]), neg_magic), mul2(ws0p, as2));
+                fma2_acc(acc23[t], add2(pack2i(d[2], d[3]), neg_magic), mul2(ws1p, as2));
+            }
+        }
+    };
+#pragma unroll 1
+    for (int g = first; g < groups; g += stride) {
+#pragma unroll
+        for (int t = 0; t < NTG; ++t) acc01[t] = acc23[t] = 0ull;
+#pragma unroll 1
+        for (int kt = 0;; kt += 2 * U) {
+            // the batch after w0's: of this row-group or the first one of the next
+            if (kt + U < Kt) load(w1, s1, g, kt + U);
+            else if (g + stride < groups) load(w1, s1, g + stride, 0);
+            batch(w0, s0, kt);
+            if (kt + U >= Kt) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) { w0[u][0] = w1[u][0]; w0[u][1] = w1[u][1]; }
+                s0 = s1;
+                break;
+            }
+            if (kt + 2 * U < Kt) load(w0, s0, g, kt + 2 * U);
+            else if (g + stride < groups) load(w0, s0, g + stride, 0);
+            batch(w1, s1, kt + U);
+            if (kt + 2 * U >= Kt) break;
+        }
+        const size_t row = (size_t)g * 16 + r;
+#pragma unroll
+        for (int t = 0; t < NTG; ++t) {
+            float o[4];
+            unpack2(acc01[t], o[0], o[1]);
+            unpack2(acc23[t], o[2], o[3]);
+            const size_t tok = (size_t)tok0 + t * 8 + 2 * c;
+            y[tok * M + row] = o[0];
+            y[(tok + 1) * M + row] = o[1];
+            y[tok * M + row + 8] = o[2];
+            y[(tok + 1) * M + row + 8] = o[3];
+        }
+    }
+}
+
 int g_sms = 0;
 int sms() {
     if (!g_sms) {
@@ -164,6 +287,40 @@ void launch_gemv_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t
 
 void launch_gemm_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t *aq,
                       const float *as, float *y, int M, int K, int T) {
+    // The staged kernel, with as many of the tokens on a warp as divide them and fit (the weights are read and
+    // their scales expanded once for all), where the copies' alignment allows.
+    const int groups = M / 16, tgroups = T / 8, Kt = K / 32;
+    int ntg = tgroups % 4 == 0 ? 4 : tgroups % 2 == 0 ? 2 : 1;
+    while (ntg > 1 && (size_t)Kt * ntg * kSActTile > kSSmem) ntg >>= 1;
+    const int windows = tgroups / ntg;
+    if (groups > 0 && windows > 0 && windows <= sms() && (size_t)Kt * ntg * kSActTile <= kSSmem &&
+        !((uintptr_t)aq & 15) && !((uintptr_t)codes & 7) && !(((uintptr_t)scales | (uintptr_t)as) & 3)) {
+        const int ctas = std::min(groups, sms() / windows), per = (groups + ctas - 1) / ctas;
+        const int rounds = (per + kWide - 1) / kWide, nw = std::max(8, (per + rounds - 1) / rounds);
+        auto go = [&](auto kernel) {
+            static const void *done[6];      // kernels of one type: by address
+            for (const void *&d : done) {
+                if (d == (const void *)kernel) break;
+                if (d) continue;
+                TQ_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSSmem));
+                d = (const void *)kernel;
+                break;
+            }
+            launch_pdl(kernel, dim3(ctas, windows), dim3(nw * 32), (size_t)Kt * ntg * kSActTile, codes, scales, aq, as,
+                       y, M, Kt, T);
+        };
+        if (nw <= kNarrow) {
+            if (ntg == 4) go(gemm_w8a8_staged_kernel<4, 4, kNarrow>);
+            else if (ntg == 2) go(gemm_w8a8_staged_kernel<2, 4, kNarrow>);
+            else go(gemm_w8a8_staged_kernel<1, 4, kNarrow>);
+        } else {
+            if (ntg == 4) go(gemm_w8a8_staged_kernel<4, 2, kWide>);
+            else if (ntg == 2) go(gemm_w8a8_staged_kernel<2, 2, kWide>);
+            else go(gemm_w8a8_staged_kernel<1, 4, kWide>);
+        }
+        TQ_LAUNCH_CHECK("gemm_w8a8_staged_kernel");
+        return;
+    }
     const long tasks = (long)(M / 16) * (T / 8);
     if (tasks <= 0) return;
     const int grid = (int)std::min<long>((tasks + kGW - 1) / kGW, 16L * sms());
