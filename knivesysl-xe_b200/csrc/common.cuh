@@ -205,6 +205,10 @@ void launch_gemm_mma(const GemmArgs &a);
 bool gemm_stream_covers(const GemmArgs &a);
 bool gemm_ring_covers(const GemmArgs &a);     // the T = 8 ring kernel takes the call
 void launch_gemm_stream(const GemmArgs &a);
+void split_scratch(size_t part_floats, int count_n, float *&part, int *&count);   // of the split reduction
+// gemm_batch.cu
+struct RingShape { int ntg, nw, per, rounds; };      // the ring kernel's plan for a call
+bool launch_gemm_batch(const GemmArgs &a, int sms, const RingShape *ring);   // false: not this kernel's call
 // gemm_dtc.cu (decode batches on tcgen05: one segment per weight, 8 <= T <= 64)
 bool gemm_dtc_covers(const GemmArgs &a);
 void launch_gemm_dtc(const GemmArgs &a);

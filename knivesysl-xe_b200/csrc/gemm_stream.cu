@@ -892,6 +892,16 @@ void ensure_scratch(size_t part_floats, int count_n) {
     }
 }
 
+}  // namespace
+
+void split_scratch(size_t part_floats, int count_n, float *&part, int *&count) {
+    ensure_scratch(part_floats, count_n);
+    part = g_scratch.part;
+    count = g_scratch.count;
+}
+
+namespace {
+
 template <int NTG, bool STAGED, bool DUMP, int kW>
 void launch_variant(const GemmArgs &a, size_t smem) {
     static bool attr_set = false;
@@ -983,7 +993,7 @@ int window_groups(const GemmArgs &a) {
 // The ring kernel takes T = 8 calls whose split activations fit beside the rings.
 // Launch shape of the ring kernel for a call, or false when the call is not its to take.
 struct RingPlan {
-    int grid, nw, ns, nwin, ntg, rounds;      // rounds: tasks that the busiest warp does one after the other
+    int grid, nw, ns, nwin, ntg, per, rounds;      // tasks of the busiest CTA, and of its busiest warp one after the other
     size_t smem;
 };
 // Plan with `ntg` token groups per warp (token windows of 8 ntg tokens on CTA columns).
@@ -1000,6 +1010,7 @@ bool ring_plan_ntg(const GemmArgs &a, int ntg, RingPlan &p) {
     // shared memory they leave goes into deeper rings (each warp's chain is then longer
     // than the memory latency its ring covers with two stages).
     const int per_cta = (groups + p.grid / S - 1) / (p.grid / S);      // tasks of the busiest CTA
+    p.per = per_cta;
     p.nw = kRW;
     if (per_cta < kRW) p.nw = std::max(8, (per_cta + 1) / 2 * 2);
     // k-tiles of the longest split (per-token splits cut whole weight-scale groups)
@@ -1120,6 +1131,12 @@ bool gemm_ring_covers(const GemmArgs &a) {
 }
 
 void launch_gemm_stream(const GemmArgs &a) {
+    if (a.T >= 16) {
+        RingPlan plan{};
+        const bool ring = ring_plan(a, plan);
+        const RingShape shape = {plan.ntg, plan.nw, plan.per, plan.rounds};
+        if (launch_gemm_batch(a, g_num_sms, ring ? &shape : nullptr)) return;
+    }
     if (launch_ring(a)) return;
     for (int i = 0; i < a.count; ++i)
         if (a.ld[i] && a.ld[i] != a.M[i]) {      // only the ring kernel strides its output rows
