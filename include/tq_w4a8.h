@@ -302,6 +302,10 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum);
  * not the sums of the codes (only where the weight has zero points), else 0; waits for the
  * stream. -1: no such call yet. */
 int qwn_dbg_prefill_sums_variant(void);
+/* How qwn_x_gemm_w8a8 runs on a GPU of `sms` SMs (host only; buffers aligned): out[0] groups of 8
+ * tokens a warp (0: the general kernel, the rest is 0 then), out[1] windows of that many groups, out[2] CTAs a window,
+ * out[3] warps a CTA, out[4] rounds of row-groups. -1: bad sizes. */
+int qwn_dbg_head_plan(int M, int K, int T, int sms, int *out);
 
 /* Model-free forms of the reference's self-checks and micro-benches
  * (xpu/src/kernels_dpas.cpp:2146-2333, 2613-2693): they take a weight record instead of

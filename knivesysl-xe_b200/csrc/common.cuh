@@ -266,6 +266,8 @@ void launch_w8_repack(const uint8_t *d_payload, const float *d_bs, int scale_col
                       uint8_t *d_codes, uint16_t *d_scales);
 void launch_gemv_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t *q,
                       const float *as, const float *residual, float *y, int M, int K, int splits);
+struct HeadPlan { int ntg, windows, ctas, warps, rounds; double clocks; };     // ntg 0: the general kernel
+HeadPlan head_plan(int groups, int tgroups, int Kt, int sms);
 void launch_gemm_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t *aq,
                       const float *as, float *y, int M, int K, int T);
 

@@ -1119,4 +1119,12 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum) {
 
 int qwn_dbg_prefill_sums_variant(void) { return tq::prefill_sums_variant(); }
 
+int qwn_dbg_head_plan(int M, int K, int T, int sms, int *out) {
+    if (!out || M <= 0 || K <= 0 || T <= 0 || (T % 8) || sms <= 0) return -1;
+    const tq::HeadPlan p = tq::head_plan(M / 16, T / 8, K / 32, sms);
+    const int v[5] = {p.ntg, p.windows, p.ctas, p.warps, p.rounds};
+    memcpy(out, v, sizeof v);
+    return 0;
+}
+
 }  // extern "C"

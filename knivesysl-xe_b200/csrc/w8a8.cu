@@ -11,10 +11,13 @@
 // megabytes, so ramp and tail do not matter. The general GEMM gives a warp one (row-group, eight
 // tokens) task, as the reference does, on mma.sync m16n8k32: its A fragment is word c and
 // word 4 + c of rows r and r + 8 of the tile, read straight from global memory. It is left for
-// activations that do not fit in shared memory (K above 25,800) and for unaligned buffers.
+// activations that do not fit in shared memory (K above 25,800), for unaligned buffers and where its plan costs
+// less (head_plan).
 #include "stream.cuh"
 
 #include <algorithm>
+#include <cmath>
+#include <type_traits>
 
 namespace tq {
 
@@ -143,17 +146,18 @@ gemm_w8a8_kernel(const uint8_t *__restrict__ codes, const uint16_t *__restrict__
 // What bounded the kernel above at 8 tokens was not the weight stream but its reads of the activations: every
 // warp of an SM comes to a k-tile's 256 bytes at about the same time and waits out an L2 latency for them. Here
 // one CTA per SM and window stages them once; a warp walks row-groups and keeps two register batches of U k-tiles
-// of its weight stream, the first one requested before the wait for the staging kernel. W = 28 warps
-// (72 registers) carry the 27.7 row-groups per SM of a 65536-row head in one round; with few row-groups
-// 16 warps with room for twice the tiles and no spills are faster (20000 x 2048, 8 tokens: 18.5 against 22.2 us
-// with 28; 65536 x 5120: 79.9 against 62.6). us of the whole call, kernel above / this one:
-// 65536 x 5120 at 8 / 16 / 32 tokens 69 / 113 / 226 -> 62 / 67 / 93; 20000 x 2048 22 / 26 / 45 -> 18 / 18 / 22;
-// 8192 x 5120 at 32 tokens 52 -> 41.
+// of its weight stream, the first one requested before the wait for the staging kernel. The last window of a
+// call may hold fewer than NTG groups of tokens (RAGGED, a form of its own: the test costs two groups a warp 7 %): its
+// warps multiply what lies in shared memory for the others and do not store it. head_plan() chooses NTG and the warps.
+// W = 28 warps (72 registers) carry the 27.7 row-groups per SM of a 65536-row head in one round; 16 warps have
+// registers for twice the tiles (20000 x 2048, 8 tokens: 18.5 against 22.2 us with 28). us of the launch alone, weights from
+// HBM, kernel above / this one: 65536 x 5120 at 8 / 16 / 24 / 32 / 48 / 64 tokens 66 / 108 / 160 / 218 / 318 / 422 -> 58 / 63 / 95 /
+// 92 / 169 / 170; 20000 x 5120 at 8 / 24 / 48 tokens 53 / 57 / 110 -> 38 / 45 / 56.
 constexpr int kSActTile = 256 + 32;        // staged codes and scales of a k-tile and eight tokens
 constexpr size_t kSSmem = 227 * 1024;
 constexpr int kWide = 28, kNarrow = 16;    // warps per CTA
 
-template <int NTG, int U, int W>
+template <int NTG, int U, int W, bool RAGGED = false>
 __global__ void __launch_bounds__(W * 32, 1)
 gemm_w8a8_staged_kernel(const uint8_t *__restrict__ codes, const uint16_t *__restrict__ scales,
                         const int8_t *__restrict__ aq, const float *__restrict__ as,
@@ -162,6 +166,7 @@ gemm_w8a8_staged_kernel(const uint8_t *__restrict__ codes, const uint16_t *__res
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int r = lane >> 2, c = lane & 3;
     const int groups = M / 16, tok0 = blockIdx.y * (8 * NTG);
+    const int real = RAGGED ? min(NTG, T / 8 - (int)blockIdx.y * NTG) : NTG;
     const int first = blockIdx.x + gridDim.x * warp, stride = gridDim.x * nw;
     // Lane (r, c) holds k = 8c..8c+7 of rows r and r + 8 as the fragment's two k positions, and takes the
     // same bytes of token r: a 32-byte row is one 8-byte load of four lanes.
@@ -185,13 +190,15 @@ gemm_w8a8_staged_kernel(const uint8_t *__restrict__ codes, const uint16_t *__res
     const uint32_t act = smem_u32(smem);
     for (int i = threadIdx.x; i < Kt * NTG * 16; i += blockDim.x) {       // 16 bytes of codes each
         const int kt = i / (NTG * 16), rem = i - kt * (NTG * 16);
-        cp_async16_plain(act + (uint32_t)(kt * NTG + (rem >> 4)) * kSActTile + (rem & 15) * 16,
-                         aq + ((size_t)kt * T + tok0) * 32 + rem * 16);
+        if (!RAGGED || (rem >> 4) < real)
+            cp_async16_plain(act + (uint32_t)(kt * NTG + (rem >> 4)) * kSActTile + (rem & 15) * 16,
+                             aq + ((size_t)kt * T + tok0) * 32 + rem * 16);
     }
     for (int i = threadIdx.x; i < Kt * NTG * 8; i += blockDim.x) {        // one scale each
         const int kt = i / (NTG * 8), rem = i - kt * (NTG * 8);
-        cp_async4(act + (uint32_t)(kt * NTG + (rem >> 3)) * kSActTile + 256 + (rem & 7) * 4,
-                  as + (size_t)kt * T + tok0 + rem);
+        if (!RAGGED || (rem >> 3) < real)
+            cp_async4(act + (uint32_t)(kt * NTG + (rem >> 3)) * kSActTile + 256 + (rem & 7) * 4,
+                      as + (size_t)kt * T + tok0 + rem);
     }
     cp_async_commit();
     cp_async_wait<0>();
@@ -249,6 +256,7 @@ gemm_w8a8_staged_kernel(const uint8_t *__restrict__ codes, const uint16_t *__res
         const size_t row = (size_t)g * 16 + r;
 #pragma unroll
         for (int t = 0; t < NTG; ++t) {
+            if (RAGGED && t >= real) break;
             float o[4];
             unpack2(acc01[t], o[0], o[1]);
             unpack2(acc23[t], o[2], o[3]);
@@ -285,20 +293,50 @@ void launch_gemv_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t
     TQ_LAUNCH_CHECK("gemv_w8a8_kernel");
 }
 
+// How a call of `groups` row-groups, `tgroups` groups of 8 tokens and Kt k-tiles runs: the plan whose busiest SM
+// needs the fewest clocks for a k-tile of all its rounds of row-groups. A round of the staged kernel is bound by latency,
+// so it costs much the same with few row-groups as with many. Measured on 65536 x 5120 and 57 other weights of 1040 to
+// 262144 rows, 8 to 2400 tokens: 475 to 505 clocks with one group of tokens a warp, 580 to 630 with two, 760 to 990 with
+// four on 17 to 28 warps; 370 to 470, 400 to 490 and 550 to 600 on up to 16; with one or two windows at least the weight
+// stream, 25 or 20 clocks a warp. The general kernel holds 32 tasks an SM: about 500 clocks a round of them and 8 a task,
+// 27.5 a task where the weights serve 8 tokens only. It is left the heads that are one round of its own and two
+// of the staged kernel (66,320 to 75,776 rows, 8 tokens: 66320 x 5120 67 us against 78), and long K, where few groups
+// fit and many windows leave SMs idle. An odd number of token groups is no reason for windows of one: 65536 x 5120, 24
+// tokens 150 us so and 95 in a window of four, 600 tokens 5810 (75 windows, one CTA each; 4110 in the general kernel) and
+// 1740. Over those calls no choice was more than 2 % behind the general kernel.
+HeadPlan head_plan(int groups, int tgroups, int Kt, int sms) {
+    HeadPlan best{};
+    if (groups <= 0 || tgroups <= 0) return best;
+    const double tasks = (double)groups * tgroups / sms;      // of an SM
+    for (int ntg = 4; ntg >= 1; ntg >>= 1) {
+        const int windows = (tgroups + ntg - 1) / ntg;
+        if ((size_t)Kt * ntg * kSActTile > kSSmem || windows > sms || (ntg > 1 && 2 * tgroups <= ntg)) continue;
+        HeadPlan p{ntg, windows, std::min(groups, sms / windows), 0, 0, 0.0};
+        const int per = (groups + p.ctas - 1) / p.ctas;
+        p.rounds = (per + kWide - 1) / kWide;
+        p.warps = std::max(8, (per + p.rounds - 1) / p.rounds);
+        double round;
+        if (p.warps > kNarrow)
+            round = ntg == 4 ? 400 + 21 * p.warps
+                  : ntg == 2 ? (windows <= 2 ? 565 : 545) + 2.5 * p.warps : windows <= 2 ? 505 : 475;
+        else
+            round = ntg == 4 ? 590 : (ntg == 2 ? 410 : 375) + (windows == 1 ? 80 : windows == 2 ? 20 : 0);
+        if (windows <= 2) round = std::max(round, (windows == 1 ? 25.0 : 20.0) * p.warps);
+        p.clocks = p.rounds * round * (tgroups % ntg ? 1.04 : 1.0);
+        if (!best.ntg || p.clocks < best.clocks) best = p;
+    }
+    const double general = std::max(500 * std::ceil(tasks / 32) + 8 * tasks, tgroups == 1 ? 27.5 * tasks : 0.0);
+    if (best.ntg && best.clocks > general) best = HeadPlan{};
+    return best;
+}
+
 void launch_gemm_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t *aq,
                       const float *as, float *y, int M, int K, int T) {
-    // The staged kernel, with as many of the tokens on a warp as divide them and fit (the weights are read and
-    // their scales expanded once for all), where the copies' alignment allows.
-    const int groups = M / 16, tgroups = T / 8, Kt = K / 32;
-    int ntg = tgroups % 4 == 0 ? 4 : tgroups % 2 == 0 ? 2 : 1;
-    while (ntg > 1 && (size_t)Kt * ntg * kSActTile > kSSmem) ntg >>= 1;
-    const int windows = tgroups / ntg;
-    if (groups > 0 && windows > 0 && windows <= sms() && (size_t)Kt * ntg * kSActTile <= kSSmem &&
-        !((uintptr_t)aq & 15) && !((uintptr_t)codes & 7) && !(((uintptr_t)scales | (uintptr_t)as) & 3)) {
-        const int ctas = std::min(groups, sms() / windows), per = (groups + ctas - 1) / ctas;
-        const int rounds = (per + kWide - 1) / kWide, nw = std::max(8, (per + rounds - 1) / rounds);
+    const int Kt = K / 32;
+    const HeadPlan p = head_plan(M / 16, T / 8, Kt, sms());
+    if (p.ntg && !((uintptr_t)aq & 15) && !((uintptr_t)codes & 7) && !(((uintptr_t)scales | (uintptr_t)as) & 3)) {
         auto go = [&](auto kernel) {
-            static const void *done[6];      // kernels of one type: by address
+            static const void *done[10];      // kernels of one type: by address
             for (const void *&d : done) {
                 if (d == (const void *)kernel) break;
                 if (d) continue;
@@ -306,18 +344,23 @@ void launch_gemm_w8a8(const uint8_t *codes, const uint16_t *scales, const int8_t
                 d = (const void *)kernel;
                 break;
             }
-            launch_pdl(kernel, dim3(ctas, windows), dim3(nw * 32), (size_t)Kt * ntg * kSActTile, codes, scales, aq, as,
-                       y, M, Kt, T);
+            launch_pdl(kernel, dim3(p.ctas, p.windows), dim3(p.warps * 32), (size_t)Kt * p.ntg * kSActTile, codes,
+                       scales, aq, as, y, M, Kt, T);
         };
-        if (nw <= kNarrow) {
-            if (ntg == 4) go(gemm_w8a8_staged_kernel<4, 4, kNarrow>);
-            else if (ntg == 2) go(gemm_w8a8_staged_kernel<2, 4, kNarrow>);
-            else go(gemm_w8a8_staged_kernel<1, 4, kNarrow>);
-        } else {
-            if (ntg == 4) go(gemm_w8a8_staged_kernel<4, 2, kWide>);
-            else if (ntg == 2) go(gemm_w8a8_staged_kernel<2, 2, kWide>);
-            else go(gemm_w8a8_staged_kernel<1, 4, kWide>);
-        }
+        auto pick = [&](auto ragged) {
+            constexpr bool R = decltype(ragged)::value;
+            if (p.warps <= kNarrow) {
+                if (p.ntg == 4) go(gemm_w8a8_staged_kernel<4, 4, kNarrow, R>);
+                else if (p.ntg == 2) go(gemm_w8a8_staged_kernel<2, 4, kNarrow, R>);
+                else go(gemm_w8a8_staged_kernel<1, 4, kNarrow>);
+            } else {
+                if (p.ntg == 4) go(gemm_w8a8_staged_kernel<4, 2, kWide, R>);
+                else if (p.ntg == 2) go(gemm_w8a8_staged_kernel<2, 2, kWide, R>);
+                else go(gemm_w8a8_staged_kernel<1, 4, kWide>);
+            }
+        };
+        if (T / 8 % p.ntg) pick(std::true_type{});
+        else pick(std::false_type{});
         TQ_LAUNCH_CHECK("gemm_w8a8_staged_kernel");
         return;
     }

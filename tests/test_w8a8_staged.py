@@ -1,7 +1,7 @@
 """int8 output head on decode batches (csrc/w8a8.cu): the kernel that stages a window's activations in
 shared memory, in all its forms (8, 16 or 32 tokens a warp, 16 or 28 warps), at tails of its register
-batches and in several rounds of row-groups, and the general kernel where the activations do not fit
-or do not allow the copies. Every output word equals the oracle's: the dots are exact integers and the
+batches, in several rounds of row-groups and with a last window that is not full, and the general kernel where the
+activations do not fit or do not allow the copies, or where it is the faster one. Every output word equals the oracle's: the dots are exact integers and the
 fp32 sums keep the order of the k-tiles."""
 import ctypes as C
 
@@ -15,11 +15,38 @@ CASES = [
     (1040, 288, 600, 0),                                               # more tokens than a decode batch
     (32, 25856, 8, 0), (32, 12960, 16, 0),                             # too long to stage; staged one group at a time
     (272, 416, 16, 4),                                                 # activations off 16 bytes
+    (66320, 96, 8, 0),                                                 # two rounds against one of the general kernel
 ]
+# M, K, tokens: groups of 8 tokens a warp, windows, CTAs a window, warps, rounds on 148 SMs, where the last window
+# is not full
+RAGGED = {
+    (38400, 96, 24): (4, 1, 148, 17, 1), (20000, 224, 56): (4, 2, 74, 17, 1), (66320, 160, 40): (4, 2, 74, 19, 3),
+    (32000, 160, 24): (4, 1, 148, 14, 1), (8192, 416, 104): (4, 4, 37, 14, 1),
+    (8192, 288, 40): (2, 3, 49, 11, 1), (20000, 96, 40): (2, 3, 49, 26, 1),
+}
+
+
+def plan(pkg, M, K, T, sms=148):
+    out = (C.c_int * 5)()
+    assert pkg.load().qwn_dbg_head_plan(M, K, T, sms, out) == 0
+    return tuple(out)
+
+
+def test_plans(pkg):
+    for case, want in RAGGED.items():
+        assert plan(pkg, *case) == want and case[2] // 8 % want[0]
+    # an odd number of token groups is no reason for windows of one group, nor many windows for idle SMs
+    for T in range(16, 2048, 8):
+        ntg, windows, ctas, warps, rounds = plan(pkg, 65536, 5120, T)
+        assert ntg > 1 and windows == -(-T // (8 * ntg)) and windows * ctas > 148 / 2 and warps <= 28
+    # 8 tokens: one round of the general kernel's tasks against two rounds of the staged one
+    assert plan(pkg, 65536, 5120, 8) == (1, 1, 148, 28, 1)
+    assert plan(pkg, 66320, 5120, 8) == plan(pkg, 75776, 5120, 8) == (0, 0, 0, 0, 0)
+    assert plan(pkg, 75792, 5120, 8) == (1, 1, 148, 17, 2)
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M,K,T,off", CASES)
+@pytest.mark.parametrize("M,K,T,off", CASES + [(*c, 0) for c in RAGGED])
 def test_head_equals_the_oracle(lib, pkg, orc, M, K, T, off):
     rng = np.random.default_rng(M + K + T)
     codes = rng.integers(-127, 128, size=M * K, dtype=np.int8)
