@@ -302,6 +302,11 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum);
  * not the sums of the codes (only where the weight has zero points), else 0; waits for the
  * stream. -1: no such call yet. */
 int qwn_dbg_prefill_sums_variant(void);
+/* Whether qwn_x_gemm_w4a8_fanout with these weights takes the kernel for decode batches (csrc/gemm_batch.cu) on
+ * a GPU of `sms` SMs (host only; buffers aligned): 1 and out[0] groups of 8 tokens a warp, out[1] 1 for the form of up to 16 warps, out[2]
+ * warps a CTA, out[3] rounds of tasks, out[4] splits, out[5] phases of the K range, out[6] k-tiles of one; 0: another
+ * kernel's call; -1: bad sizes. */
+int qwn_dbg_batch_plan(const int *rows, int count, int K, int T, int k64, int sms, int *out);
 /* How qwn_x_gemm_w8a8 runs on a GPU of `sms` SMs (host only; buffers aligned): out[0] groups of 8
  * tokens a warp (0: the general kernel, the rest is 0 then), out[1] windows of that many groups, out[2] CTAs a window,
  * out[3] warps a CTA, out[4] rounds of row-groups. -1: bad sizes. */

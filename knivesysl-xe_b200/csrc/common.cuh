@@ -207,8 +207,19 @@ bool gemm_ring_covers(const GemmArgs &a);     // the T = 8 ring kernel takes the
 void launch_gemm_stream(const GemmArgs &a);
 void split_scratch(size_t part_floats, int count_n, float *&part, int *&count);   // of the split reduction
 // gemm_batch.cu
-struct RingShape { int ntg, nw, per, rounds; };      // the ring kernel's plan for a call
-bool launch_gemm_batch(const GemmArgs &a, int sms, const RingShape *ring);   // false: not this kernel's call
+// The plan of the kernel that a call goes to otherwise: the streaming kernel; the ring kernel with windows of 8 tokens on
+// up to 20 warps with four ring stages each, or on more warps or fewer stages; or with several token groups a warp.
+// Token groups a warp, warps, tasks of the busiest CTA, k-tiles of the longest split.
+struct RingShape {
+    enum Kernel { kStream, kSmall, kLarge, kSeveral } kernel;
+    int ntg, warps, per, span;
+};
+// This kernel's: token groups a warp, 16 warps at most instead of 12, CTAs a split, tasks of the busiest, its warps and
+// their rounds of tasks, k-tiles of the longest split, of a phase (P), and phases.
+struct BatchPlan { int ntg, wide, ctas, per, warps, rounds, span, P, phases; double clocks; };
+bool batch_plan(const GemmArgs &a, int sms, const RingShape &other, BatchPlan &plan);   // false: the other kernels' call
+bool decode_batch_plan(const GemmArgs &a, int sms, BatchPlan &plan);     // the same, against their plan (gemm_stream.cu)
+bool launch_gemm_batch(const GemmArgs &a, int sms, const RingShape &other);   // false: not this kernel's call
 // gemm_dtc.cu (decode batches on tcgen05: one segment per weight, 8 <= T <= 64)
 bool gemm_dtc_covers(const GemmArgs &a);
 void launch_gemm_dtc(const GemmArgs &a);

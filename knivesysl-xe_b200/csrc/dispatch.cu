@@ -1119,6 +1119,28 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum) {
 
 int qwn_dbg_prefill_sums_variant(void) { return tq::prefill_sums_variant(); }
 
+int qwn_dbg_batch_plan(const int *rows, int count, int K, int T, int k64, int sms, int *out) {
+    if (!rows || !out || count < 1 || count > 4 || K <= 0 || (K % 32) || T <= 0 || (T % 8) || sms <= 0) return -1;
+    tq::GemmArgs a{};
+    a.K = K;
+    a.T = T;
+    a.ksh = k64 ? 1 : 0;
+    a.count = count;
+    a.max_splits = 1;
+    for (int i = 0; i < count; ++i) {
+        int ms = 1;
+        if (rows[i] <= 0 || rows[i] % 16 || tq::build_segments(rows[i] / 16, K / 32, T, nullptr, 0, a.seg[i], ms)) return -1;
+        a.M[i] = rows[i];
+        a.goff[i + 1] = a.goff[i] + rows[i] / 16;
+        a.max_splits = std::max(a.max_splits, ms);
+    }
+    tq::BatchPlan p;
+    if (!tq::gemm_stream_covers(a) || !tq::decode_batch_plan(a, sms, p)) return 0;
+    const int v[7] = {p.ntg, p.wide, p.warps, p.rounds, a.max_splits, p.phases, p.P};
+    memcpy(out, v, sizeof v);
+    return 1;
+}
+
 int qwn_dbg_head_plan(int M, int K, int T, int sms, int *out) {
     if (!out || M <= 0 || K <= 0 || T <= 0 || (T % 8) || sms <= 0) return -1;
     const tq::HeadPlan p = tq::head_plan(M / 16, T / 8, K / 32, sms);

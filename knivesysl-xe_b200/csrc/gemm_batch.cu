@@ -17,11 +17,13 @@
 //  * at most 12 (168 registers) or 16 warps (128), so that the chains of a warp's units can overlap.
 // Arithmetic, order of the sums and the split reduction are those of gemm_stream.cu.
 //
-// What bounds it: a warp's instructions at 2 to 3.5 clocks each (32 a unit of 16 x 8 x 32 at NTG 2, 24 at 4;
-// 9 warps on four schedulers use 47 % of the issue slots). us per call with the staging, before / now:
-// 5120 x 17408 K32 at 64 / 24 / 16 tokens 110.5 / 40.9 / 30.2 -> 98.7 / 36.4 / 27.7; 17408 x 17408 at 64 267 -> 196;
-// 4096 x 4096 at 64 32.6 -> 23.6; 2048 x 8192 K64 at 64 34.3 -> 25.1; 17408 x 5120 K64 at 48 58.4 -> 46.6; three of
-// 6000 x 6016 at 24 48.3 -> 35.2; 704 x 8992 at 64 36.5 -> 18.8.
+// What bounds it: the latency between a warp's instructions (32 a unit of 16 x 8 x 32 at NTG 2, 24 at 4). At 64 tokens on
+// 5120 x 17408 an SM has nine warps, 2.25 a scheduler, each 4.7 clocks from one instruction to the next: 47 % of the issue
+// slots. us of the launch alone, weights from HBM, the kernels before / this one: 5120 x 17408 K32 at 64 / 24 / 16 tokens
+// 104.5 / 34.0 / 25.3 -> 92.0 / 30.7 / 23.6; 17408 x 17408 at 64 252 -> 172; 4096 x 4096 at 64 23.7 -> 18.6; 2048 x 8192
+// K64 at 64 / 16 26.5 / 11.2 -> 20.9 / 8.5; 17408 x 5120 K64 at 48 52.9 -> 41.9; three of 6000 x 6016 at 24 43.9 -> 31.2;
+// 704 x 8992 at 64 26.6 -> 11.1. (The first of them is not what the kernel is for: windows of 8 tokens on 18 warps, a form
+// of the ring kernel that was not built in, came to the same time there.)
 // Tried without gain: {ws, ws, z, z} in the scale buffer instead of pairs built from two words (105 against 99 us
 // at 64 tokens: the reads' latency), 20 warps of 96 registers (126).
 #include "stream.cuh"
@@ -301,76 +303,99 @@ gemm_w4a8_batch_kernel(const GemmArgs a, const BatchArgs b, float *__restrict__ 
 
 }  // namespace
 
-// Plans are compared by the clocks that the busiest SM's schedulers need for a k-tile of its warps. A warp issues
-// about 40 + 12 NTG instructions a k-tile here, 27 + 11 NTG in the ring kernel; with one warp on a scheduler an
-// instruction takes 3.3 clocks, with more of them the scheduler is shared (kShare, fitted to the calls of the
-// comment on top and forty more). With several groups a warp the ring kernel takes 5.5 clocks and more an
-// instruction (fewer registers, shorter look-ahead); with windows of 8 tokens it is not bound by instructions
-// but takes 13.5 clocks a (warp, k-tile) of the SM. Split calls cost it another 15,000 clocks. Over those calls
-// the choice is at most 6 % behind the faster kernel, 3 % where that is the ring kernel.
+// Which kernel: both plans are turned into clocks of the busiest SM for the call, and the smaller one is taken, the
+// other kernel's unless this kernel's is 4.5 % below it. (The other kernel is the ring kernel, or the streaming kernel where the
+// activations of 8 tokens do not fit beside the rings: a split of more than 266 k-tiles.) The terms are what the
+// kernels are made of: per k-tile, what a unit of one (row-group, token groups) costs by the warps that share an SM; the
+// rounds of a warp's tasks, the last one with the warps that it has; launch and staging; the phases; with splits, the
+// partials and their ordered sum, again for each further round.
+// The constants are on one scale with each other rather than clocks: they minimise the time of the kernels chosen, with
+// a penalty where that is this one and it loses against the other, over 3500 calls drawn from 128 to 17408 rows,
+// one to four weights, K 512 to 17408, both scale groups and 16 to 64 tokens, every plan measured. There the calls run
+// in 0.80 of the other kernel's time, 0.2 % above the best plan of each; 15 are more than 3 % behind the other kernel, two more
+// than 8 %, and of 440 calls that the constants had not seen four, the worst by 9 %. Counting a warp's instructions alone, without the sums of the splits and the rounds, left 243 of them more
+// than 3 % behind, one by 46 % (912 x 6464 K64, 40 tokens: 13.3 us against 9.2).
 namespace {
 
-constexpr double kShare[5] = {0.0, 3.3, 4.2, 5.6, 6.6};
-double shared_clocks(int warps) {
-    const int k = (warps + 3) / 4;
-    return k <= 4 ? kShare[k] : 6.6 + (k - 4);
+constexpr double kLead = 1.045;
+
+// rounds of `per` tasks on `warps` warps: the clocks of a k-tile in all of them
+template <typename F>
+double all_rounds(int per, int warps, F clocks) {
+    return per / warps * clocks(warps) + (per % warps ? clocks(per % warps) : 0.0);
 }
 
-struct BatchPlan {
-    int ntg, wide, ctas, nw;      // token groups per warp; 16 warps instead of 12; CTAs per split; warps
-    double clocks;
-};
-
-BatchPlan batch_plan(const GemmArgs &a, int sms) {
-    const int tg = a.T / 8, groups = a.goff[a.count];
-    BatchPlan best{};
-    for (int ntg = 8; ntg >= 1; --ntg) {
-        if (tg % ntg || (ntg == 1 && tg > 1)) continue;
-        for (int wide = 0; wide <= (ntg <= 4 ? 1 : 0); ++wide) {
-            const long tasks = (long)groups * (tg / ntg);
-            BatchPlan p{ntg, wide, 0, 0, 0.0};
-            p.ctas = (int)std::max(1L, std::min<long>(sms / a.max_splits, tasks));
-            const int per = (int)((tasks + p.ctas - 1) / p.ctas), most = wide ? 16 : 12;
-            const int rounds = (per + most - 1) / most;
-            p.nw = std::max(4, (per + rounds - 1) / rounds);
-            p.clocks = rounds * (40 + 12 * ntg) * shared_clocks(p.nw) * (wide ? 1.1 : 1.0);
-            if (!best.ntg || p.clocks < best.clocks) best = p;
+double other_clocks(const RingShape &r, int splits) {
+    const double unit = all_rounds(r.per, r.warps, [&](int w) {
+        switch (r.kernel) {
+            case RingShape::kStream: return std::max(180.0, (r.ntg == 1 ? 18.6 : 30.0) * w);
+            case RingShape::kSmall: return 18.6 * w + 8;
+            case RingShape::kLarge: return 12.4 * w + 116;
+            default: return (16 + 19 * r.ntg) * std::max(4.6, 0.38 * w);
         }
-    }
-    return best;
+    });
+    static const double lead_in[4] = {2800, 4200, 4000, 8200};
+    const bool one = r.ntg == 1, wide = r.kernel == RingShape::kSeveral;
+    const double sums = splits == 1 ? 0.0 : !one ? 2800.0 * r.ntg : r.kernel == RingShape::kLarge ? 9600.0 : 4200.0;
+    const int rounds = (r.per + r.warps - 1) / r.warps;
+    return lead_in[r.kernel] + r.span * (unit + (wide ? 19 * r.ntg : 0)) + sums + (splits > 1 ? 19000.0 * (rounds - 1) : 0);
+}
+
+double batch_clocks(const BatchPlan &p, int splits) {
+    static const double shared[4] = {4.0, 5.8, 7.9, 10.0};      // 1 to 4 warps on a scheduler
+    const double unit = all_rounds(p.per, p.warps, [&](int w) { return (19 + 10 * p.ntg) * shared[(w - 1) / 4]; });
+    // many splits on four or five warps: measured, the longer a split, without a cause that is known
+    const double few = splits >= 8 && p.warps <= 5 ? 38.0 * p.ntg * p.span : 0.0;
+    const int passes = p.phases > 1 ? p.phases * p.rounds : 1;
+    return 6000 + p.span * unit + few + 4000.0 * (passes - 1) +
+           (splits > 1 ? 1200 * p.ntg + 20500 * (p.rounds - 1) + (p.wide ? 4700 * p.rounds : 0) : 0);
 }
 
 }  // namespace
 
-bool launch_gemm_batch(const GemmArgs &a, int sms, const RingShape *ring) {
+bool batch_plan(const GemmArgs &a, int sms, const RingShape &other, BatchPlan &best) {
     if (a.mode || a.x || a.dump || a.npeer || a.T < 16 || a.T > 64 || a.T % 8) return false;
-    if (((uintptr_t)a.aq | (uintptr_t)a.as | (uintptr_t)a.asum) & 15) return false;      // 16-byte copies
     for (int i = 0; i < a.count; ++i)
         if (a.ld[i] && a.ld[i] != a.M[i]) return false;
-    const int S = a.max_splits, Kt = a.K / 32, groups = a.goff[a.count];
+    const int S = a.max_splits, Kt = a.K / 32, groups = a.goff[a.count], tg = a.T / 8;
     if (S > 16 || S > sms || groups <= 0) return false;
-    const int span = (Kt + S - 1) / S;
-    const BatchPlan plan = batch_plan(a, sms);
-    if (ring) {
-        const int warps = std::min(ring->nw, ring->per);
-        const double clocks = ring->rounds * (ring->ntg == 1 ? 13.5 * warps
-                                                             : (27 + 11 * ring->ntg) * std::max(5.5, 0.45 * warps));
-        if (1.05 * plan.clocks >= clocks + (S > 1 ? std::min(150.0, 15000.0 / span) : 0.0)) return false;
-        if (a.T == 16 && S > 4) return false;      // short splits (2048 x 8192: 13.6 against 13.0 us)
+    best = BatchPlan{};
+    for (int ntg = 8; ntg >= 2; --ntg) {
+        if (tg % ntg) continue;
+        const long tasks = (long)groups * (tg / ntg);
+        for (int wide = 0; wide <= (ntg == 3 || ntg == 4 ? 1 : 0); ++wide) {
+            BatchPlan p{};
+            p.ntg = ntg;
+            p.wide = wide;
+            p.ctas = (int)std::max(1L, std::min<long>(sms / S, tasks));
+            p.per = (int)((tasks + p.ctas - 1) / p.ctas);
+            if (wide && p.per <= 12) continue;
+            const int most = wide ? 16 : 12;
+            p.rounds = (p.per + most - 1) / most;
+            p.warps = std::max(4, (p.per + p.rounds - 1) / p.rounds);
+            p.span = (Kt + S - 1) / S;
+            const size_t room = kSmemLimit - (size_t)p.warps * kExpBytes, tile = (size_t)a.T * 40;
+            p.P = (p.span + kCT - 1) / kCT * kCT;
+            p.phases = 1;
+            if (p.P * tile > room) {
+                p.P = (int)(room / 2 / tile) / kCT * kCT;
+                p.phases = (p.span + p.P - 1) / p.P;
+            }
+            p.clocks = batch_clocks(p, S);
+            if (!best.ntg || p.clocks < best.clocks) best = p;
+        }
     }
-    const int ntg = plan.ntg, nw = plan.nw, ctas = plan.ctas;
+    return best.ntg && kLead * best.clocks < other_clocks(other, S);
+}
+
+bool launch_gemm_batch(const GemmArgs &a, int sms, const RingShape &other) {
+    BatchPlan plan;
+    if (((uintptr_t)a.aq | (uintptr_t)a.as | (uintptr_t)a.asum) & 15) return false;      // 16-byte copies
+    if (!batch_plan(a, sms, other, plan)) return false;
+    const int S = a.max_splits, groups = a.goff[a.count];
+    const int ntg = plan.ntg, nw = plan.warps, ctas = plan.ctas;
     const long tasks = (long)groups * (a.T / 8 / ntg);
-    BatchArgs b{};
-    const size_t room = kSmemLimit - (size_t)nw * kExpBytes, tile = (size_t)a.T * 40;
-    const int whole = (span + kCT - 1) / kCT * kCT;
-    if (whole * tile <= room) {
-        b.P = whole;
-        b.phases = 1;
-    } else {
-        b.P = (int)(room / 2 / tile) / kCT * kCT;
-        b.phases = (span + b.P - 1) / b.P;
-    }
-    b.buf_bytes = (int)(b.P * tile);
+    const BatchArgs b = {plan.P, plan.phases, (int)(plan.P * (size_t)a.T * 40)};
     const size_t smem = (size_t)nw * kExpBytes + (size_t)b.buf_bytes * (b.phases > 1 ? 2 : 1);
     float *part = nullptr;
     int *count = nullptr;
@@ -388,7 +413,6 @@ bool launch_gemm_batch(const GemmArgs &a, int sms, const RingShape *ring) {
     };
     switch (ntg * 2 + plan.wide) {
         case 4: go(gemm_w4a8_batch_kernel<2, 12>); break;
-        case 5: go(gemm_w4a8_batch_kernel<2, 16>); break;
         case 6: go(gemm_w4a8_batch_kernel<3, 12>); break;
         case 7: go(gemm_w4a8_batch_kernel<3, 16>); break;
         case 8: go(gemm_w4a8_batch_kernel<4, 12>); break;

@@ -864,6 +864,15 @@ gemm_w4a8_ring_kernel(const GemmArgs a, float *__restrict__ part, int *__restric
 }
 
 int g_num_sms = 0;
+int num_sms() {
+    if (!g_num_sms) {
+        int dev = 0;
+        TQ_CHECK(cudaGetDevice(&dev));
+        TQ_CHECK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
+        if (g_num_sms <= 0) g_num_sms = 148;
+    }
+    return g_num_sms;
+}
 constexpr size_t kSmemLimit = 227 * 1024;
 
 // Library scratch of the split reduction: partial tiles and one arrival counter per
@@ -917,7 +926,7 @@ void launch_variant(const GemmArgs &a, size_t smem) {
     if (S > 1 && !DUMP)
         ensure_scratch((size_t)nwin * groups * S * NTG * 128, nwin * groups);
     const int want = ((groups + kW - 1) / kW) * S;
-    const int grid = std::max(S, std::min(std::max(1, g_num_sms / nwin), want));
+    const int grid = std::max(S, std::min(std::max(1, num_sms() / nwin), want));
     launch_pdl(gemm_w4a8_stream_kernel<NTG, STAGED, DUMP, kW>, dim3(grid, nwin), dim3(kW * 32),
                smem, a, g_scratch.part, g_scratch.count);
     TQ_LAUNCH_CHECK("gemm_w4a8_stream_kernel");
@@ -925,12 +934,6 @@ void launch_variant(const GemmArgs &a, size_t smem) {
 
 template <int NTG>
 void launch_ntg(const GemmArgs &a) {
-    if (!g_num_sms) {
-        int dev = 0;
-        TQ_CHECK(cudaGetDevice(&dev));
-        TQ_CHECK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
-        if (g_num_sms <= 0) g_num_sms = 148;
-    }
     if (a.dump) {
         launch_variant<NTG, false, true, 16>(a, (size_t)16 * kExpBytes);
         return;
@@ -944,7 +947,7 @@ void launch_ntg(const GemmArgs &a) {
                 // 24 warps per CTA (fewer registers each) when that saves a whole pass over
                 // the row-groups: every (row-group, split) is one indivisible warp task
                 const int groups = a.goff[a.count];
-                const int ctas = std::max(1, g_num_sms / S);
+                const int ctas = std::max(1, num_sms() / S);
                 const int rounds16 = (groups + ctas * 16 - 1) / (ctas * 16);
                 const int rounds24 = (groups + ctas * 24 - 1) / (ctas * 24);
                 if (rounds24 < rounds16 && rounds16 <= 3) {
@@ -993,16 +996,16 @@ int window_groups(const GemmArgs &a) {
 // The ring kernel takes T = 8 calls whose split activations fit beside the rings.
 // Launch shape of the ring kernel for a call, or false when the call is not its to take.
 struct RingPlan {
-    int grid, nw, ns, nwin, ntg, per, rounds;      // tasks of the busiest CTA, and of its busiest warp one after the other
+    int grid, nw, ns, nwin, ntg, per, span, rounds;      // tasks of the busiest CTA, and of its busiest warp one after the other
     size_t smem;
 };
 // Plan with `ntg` token groups per warp (token windows of 8 ntg tokens on CTA columns).
-bool ring_plan_ntg(const GemmArgs &a, int ntg, RingPlan &p) {
+bool ring_plan_ntg(const GemmArgs &a, int ntg, int sms, RingPlan &p) {
     p.ntg = ntg;
     p.nwin = a.T / (8 * ntg);                 // token windows: CTA columns (grid.y)
     const int Kt = a.K >> 5, S = a.max_splits;
     const int groups = a.goff[a.count];
-    const int ctas = g_num_sms / p.nwin;      // CTAs of one window
+    const int ctas = sms / p.nwin;            // CTAs of one window
     if (S > ctas || groups <= 0) return false;
     const long most = (long)groups * S;
     p.grid = (int)std::max<long>(S, std::min<long>(ctas - ctas % S, most));
@@ -1015,7 +1018,7 @@ bool ring_plan_ntg(const GemmArgs &a, int ntg, RingPlan &p) {
     if (per_cta < kRW) p.nw = std::max(8, (per_cta + 1) / 2 * 2);
     // k-tiles of the longest split (per-token splits cut whole weight-scale groups)
     const int Ktg = Kt >> a.ksh;
-    const int span = a.mode ? (((Ktg + S - 1) / S) << a.ksh) : (Kt + S - 1) / S;
+    const int span = p.span = a.mode ? (((Ktg + S - 1) / S) << a.ksh) : (Kt + S - 1) / S;
     const size_t fixed = kRHead + (size_t)span * ntg * kActTileBytes + (a.npeer ? (size_t)p.nw * 512 : 0);
     if (ntg > 1) {
         // several token groups per warp: one instantiation, at most 20 warps (more registers
@@ -1047,23 +1050,17 @@ int ring_cost(const RingPlan &p) { return p.rounds * (5 + 3 * p.ntg) * std::max(
 // loss against windows is 7 % (1024 x 5120, 56 tokens: 23.7 / 25.3), against one warp none.
 // The reference's arithmetic keeps the powers of two: its split rule leaves few tasks per call
 // (24 tokens 42.0 against 43.8 us on 5120 x 17408, 48 tokens 19.6 against 24.7 on 2 x 1024 x 5120).
-bool ring_plan(const GemmArgs &a, RingPlan &p) {
+bool ring_plan(const GemmArgs &a, int sms, RingPlan &p) {
     if (a.T < 8 || a.T > 64 || (a.T % 8) || a.dump) return false;
     if (a.x && (a.T != 8 || a.mode)) return false;   // the fused quantiser serves one window
-    if (!g_num_sms) {
-        int dev = 0;
-        TQ_CHECK(cudaGetDevice(&dev));
-        TQ_CHECK(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
-        if (g_num_sms <= 0) g_num_sms = 148;
-    }
     const int tg = a.T / 8;
     bool found = false;
     for (int ntg = 8; ntg >= 1 && !found; ntg >>= 1)
-        found = tg % ntg == 0 && (ntg == 1 || !a.npeer) && ring_plan_ntg(a, ntg, p);
+        found = tg % ntg == 0 && (ntg == 1 || !a.npeer) && ring_plan_ntg(a, ntg, sms, p);
     if (a.mode && !a.npeer)
         for (int ntg = 7; ntg >= 3; --ntg) {
             RingPlan wide;
-            if (tg % ntg || ntg == 4 || !ring_plan_ntg(a, ntg, wide)) continue;
+            if (tg % ntg || ntg == 4 || !ring_plan_ntg(a, ntg, sms, wide)) continue;
             if (!found || ring_cost(wide) < ring_cost(p)) {
                 p = wide;
                 found = true;
@@ -1074,7 +1071,7 @@ bool ring_plan(const GemmArgs &a, RingPlan &p) {
 
 bool launch_ring(const GemmArgs &a) {
     RingPlan plan;
-    if (!ring_plan(a, plan)) return false;
+    if (!ring_plan(a, num_sms(), plan)) return false;
     const int Kt = a.K >> 5, S = a.max_splits;
     const int groups = a.goff[a.count];
     const int grid = plan.grid, nw = plan.nw, ns = plan.ns;
@@ -1127,16 +1124,30 @@ bool launch_ring(const GemmArgs &a) {
 
 bool gemm_ring_covers(const GemmArgs &a) {
     RingPlan plan;
-    return gemm_stream_covers(a) && ring_plan(a, plan);
+    return gemm_stream_covers(a) && ring_plan(a, num_sms(), plan);
+}
+
+namespace {
+// The plan of the kernel that takes a call here, as the batch kernel compares itself with it.
+RingShape other_shape(const GemmArgs &a, int sms) {
+    RingPlan plan{};
+    if (ring_plan(a, sms, plan)) {
+        const auto kernel = plan.ntg > 1 ? RingShape::kSeveral
+                          : plan.ns == 4 && plan.nw <= 20 ? RingShape::kSmall : RingShape::kLarge;
+        return {kernel, plan.ntg, plan.nw, plan.per, plan.span};
+    }
+    const int S = a.max_splits, groups = a.goff[a.count], ntg = window_groups(a), nwin = a.T / (8 * ntg);
+    const int grid = std::max(S, std::min(std::max(1, sms / nwin), (groups + 15) / 16 * S));
+    return {RingShape::kStream, ntg, 16, (groups + grid / S - 1) / (grid / S), ((a.K >> 5) + S - 1) / S};
+}
+}  // namespace
+
+bool decode_batch_plan(const GemmArgs &a, int sms, BatchPlan &plan) {
+    return batch_plan(a, sms, other_shape(a, sms), plan);
 }
 
 void launch_gemm_stream(const GemmArgs &a) {
-    if (a.T >= 16) {
-        RingPlan plan{};
-        const bool ring = ring_plan(a, plan);
-        const RingShape shape = {plan.ntg, plan.nw, plan.per, plan.rounds};
-        if (launch_gemm_batch(a, g_num_sms, ring ? &shape : nullptr)) return;
-    }
+    if (a.T >= 16 && launch_gemm_batch(a, num_sms(), other_shape(a, num_sms()))) return;
     if (launch_ring(a)) return;
     for (int i = 0; i < a.count; ++i)
         if (a.ld[i] && a.ld[i] != a.M[i]) {      // only the ring kernel strides its output rows
