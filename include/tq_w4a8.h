@@ -302,6 +302,9 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum);
  * not the sums of the codes (only where the weight has zero points), else 0; waits for the
  * stream. -1: no such call yet. */
 int qwn_dbg_prefill_sums_variant(void);
+/* Tokens of a tile of the tensor-core prefill kernel on a GPU of `sms` SMs (host only): per_token 0 (a scale per block,
+ * 4-bit activations) 32 to 128 with tiles of 256 rows, or 256 with 128 rows; else 128, 192 or 256. -1: bad sizes. */
+int qwn_dbg_prefill_tile(int M, int T, int per_token, int sms);
 /* Whether qwn_x_gemm_w4a8_fanout with these weights takes the kernel for decode batches (csrc/gemm_batch.cu) on
  * a GPU of `sms` SMs (host only; buffers aligned): 1 and out[0] groups of 8 tokens a warp, out[1] 1 for the form of up to 16 warps, out[2]
  * warps a CTA, out[3] rounds of tasks, out[4] splits, out[5] phases of the K range, out[6] k-tiles of one; 0: another

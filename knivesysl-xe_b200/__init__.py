@@ -97,6 +97,7 @@ SIGNATURES = {
     "qwn_dbg_tile_dots_gemm": (_i, [_WP, _vp, _i, _vp]),
     "qwn_dbg_prepared_act": (_i, [_i, _vp, _vp, _vp]),
     "qwn_dbg_prefill_sums_variant": (_i, []),
+    "qwn_dbg_prefill_tile": (_i, [_i, _i, _i, _i]),
     "qwn_dbg_batch_plan": (_i, [C.POINTER(_i), _i, _i, _i, _i, _i, C.POINTER(_i)]),
     "qwn_dbg_head_plan": (_i, [_i, _i, _i, _i, C.POINTER(_i)]),
     "qwn_gemv_bench": (_d, [_WP, _i]), "qwn_gemm_bench": (_d, [_WP, _i, _i]),

@@ -264,6 +264,7 @@ struct GemmTcArgs {
 };
 int launch_gemm_tc(const GemmTcArgs &a);   // returns 0, or <0 when the shape is not covered
 int prefill_sums_variant();                // see qwn_dbg_prefill_sums_variant
+int prefill_tile_tokens(int M, int T, int sms, bool per_token);     // see qwn_dbg_prefill_tile
 
 // gemv_e2m3.cu: the scalar tier of a weight that still holds its E2M3 payload
 int launch_gemv_e2m3(const tq_qmma_weight_t *w, const float *d_x, const float *d_residual, float *d_y);

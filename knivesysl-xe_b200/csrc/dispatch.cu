@@ -1119,6 +1119,11 @@ int qwn_dbg_prepared_act(int K, int8_t *d_q, float *d_scale, int32_t *d_sum) {
 
 int qwn_dbg_prefill_sums_variant(void) { return tq::prefill_sums_variant(); }
 
+int qwn_dbg_prefill_tile(int M, int T, int per_token, int sms) {
+    if (M <= 0 || M % 128 || T < 128 || T % 8 || sms <= 0) return -1;
+    return tq::prefill_tile_tokens(M, T, sms, per_token != 0);
+}
+
 int qwn_dbg_batch_plan(const int *rows, int count, int K, int T, int k64, int sms, int *out) {
     if (!rows || !out || count < 1 || count > 4 || K <= 0 || (K % 32) || T <= 0 || (T % 8) || sms <= 0) return -1;
     tq::GemmArgs a{};

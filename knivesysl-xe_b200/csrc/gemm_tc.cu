@@ -18,8 +18,8 @@
 //
 // Mapping. Weights are the M side of the MMA (128 output rows = 128 TMEM lanes), tokens the
 // N side, and one accumulator read-out yields exactly the per-k-tile dots the reference
-// promotes. A CTA's tile is two row blocks x 32 to 128 tokens where the promote reads an activation scale
-// per token and group (block and 4-bit modes), one row block x 128, 192 or 256 tokens with per-token
+// promotes. A CTA's tile is two row blocks x 32 to 128 tokens, or one x 256, where the promote reads an activation
+// scale per token and group (block and 4-bit modes), one row block x 128, 192 or 256 tokens with per-token
 // scales (choose_tile_tokens). The K loop advances in steps of two k-tiles. Both operands come from images
 // that one pre-pass writes in the operand layout (canonical no-swizzle K-major core matrices): the
 // activation image and the weight image, every 4-bit code expanded to e4m3 q - z once per call.
@@ -102,9 +102,9 @@ template <int MODE, int WT>
 struct TcTile {
     static constexpr bool kPerTok = MODE == kToken || MODE == kToken64;
     static constexpr int GW = MODE == kInt4 || MODE == kToken64 ? 2 : 1;  // k-tiles per promote
-    static constexpr int R = kPerTok ? 1 : 2;                // row blocks of 128
+    static constexpr int R = kPerTok || WT > 32 ? 1 : 2;     // row blocks of 128
     static constexpr int TN = kWorkWarps / 4 * WT;           // tokens per tile
-    static constexpr int kChunk = R == 2 ? 8 : 16;           // tokens of one TMEM load of a worker
+    static constexpr int kChunk = kPerTok ? 16 : 8;          // tokens of one TMEM load of a worker
     static constexpr int kRest = WT % kChunk, kMain = WT - kRest;
     static constexpr int kRowCols = (TN + 31) / 32 * 32;     // accumulator columns of a row block
     static constexpr int kAccCols = R * kRowCols;            // ... of a promote group
@@ -339,6 +339,7 @@ __device__ __forceinline__ void reg_dealloc() {
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&v)[4]) { tmem_ld4(taddr, v); }
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&v)[8]) { tmem_ld8(taddr, v); }
 __device__ __forceinline__ void tmem_ldn(uint32_t taddr, uint32_t (&v)[16]) { tmem_ld16(taddr, v); }
+__device__ __forceinline__ void tmem_wait_ldn(uint32_t (&v)[8]) { tmem_wait_ld8(v); }
 __device__ __forceinline__ void tmem_wait_ldn(uint32_t (&v)[16]) { tmem_wait_ld16(v); }
 // one wait for two loads
 __device__ __forceinline__ void tmem_wait_ldn2(uint32_t (&v)[4], uint32_t (&w)[4]) { tmem_wait_ld4x2(v, w); }
@@ -558,9 +559,14 @@ __device__ __forceinline__ void tc_gemm(const TcParams &p, const unsigned gen) {
                     const uint32_t at = svg + col * 4;
                     if constexpr (R == 1) {
                         uint32_t d[N];
+                        ulonglong2 as[N / 4];
                         tmem_ldn(tcol + col, d);
+                        if constexpr (!PERTOK) {
+#pragma unroll
+                            for (int j = 0; j < N / 4; ++j) as[j] = lds_pairs(at + 16 * j);
+                        }
                         tmem_wait_ldn(d);
-                        promote(d, nullptr, at, 0, i0);
+                        promote(d, as, at, 0, i0);
                     } else {
                         uint32_t d0[N], d1[N];
                         ulonglong2 as[N / 4];
@@ -820,6 +826,7 @@ template <int MODE>
 void launch_width(const TcParams &p, int TN, int sms) {
     if constexpr (TcTile<MODE, 32>::R == 2) {
         switch (TN) {
+            case 256: launch_tile<MODE, 64>(p, sms); break;
             case 128: launch_tile<MODE, 32>(p, sms); break;
             case 112: launch_tile<MODE, 28>(p, sms); break;
             case 96: launch_tile<MODE, 24>(p, sms); break;
@@ -842,9 +849,12 @@ void launch_width(const TcParams &p, int TN, int sms) {
 // / 92 us at 32 / 48 / 64 / 80 / 96 / 112 / 128 tokens and K 5120 (0.6 us a token and 25 tokens' worth of fixed
 // cost; W4A4 0.34 and 30); with per-token scales a round of 128 rows takes 24 / 33 / 40 us at 128 / 192 / 256
 // tokens on K64 weights (57) and 44 / 56 / 67 on K32 (108). The rest is how many rounds the tiles of a
-// width need: 136 tokens on 10240 rows are one round of 48 (74 us; 64: 81, 128: 122), 1000 on 5120 rows
-// two of 80 (485; 96: 535, 128: 680). Over twelve shapes in all modes the choice is within 1 % of the
-// fastest width.
+// width need: 136 tokens on 10240 rows are one round of 48 (us of the whole call: 67; 64 tokens: 81, 128: 122), 1000 on
+// 5120 rows two of 80 (485; 96: 535, 128: 680). With one constant for both scale groups, and one for block mode and W4A4,
+// the choice is within 1 % of the fastest width over twelve shapes in all modes. In block and 4-bit mode there is one tile of a single row block too, 256 tokens wide, for calls that it takes
+// in one round and pairs do not, an odd number of row blocks most of all (4736 x 5120, 37 of them, 1024 tokens: 119
+// against 138 us in two rounds of 80, W4A4 67 against 86); 124 against 112 us where both are one round, hence its 82 units less
+// than the 256 tokens (9472 x 5120, 512 tokens).
 int choose_tile_tokens(int M, int T, int sms, bool per_token) {
     const int rows = (per_token ? 1 : 2) * kTM, widest = per_token ? 256 : 128, step = per_token ? 64 : 16;
     int best = 0;
@@ -856,6 +866,10 @@ int choose_tile_tokens(int M, int T, int sms, bool per_token) {
             best = tn;
             best_cost = cost;
         }
+    }
+    if (!per_token) {
+        const long tiles = (long)(M / kTM) * ((T + 255) / 256);
+        if ((tiles + sms - 1) / sms * (256 - 82) < best_cost) best = 256;
     }
     return best;
 }
@@ -921,6 +935,8 @@ int launch_gemm_tc(const GemmTcArgs &a) {
     TQ_LAUNCH_CHECK("gemm_w4a8_tc_kernel");
     return 0;
 }
+
+int prefill_tile_tokens(int M, int T, int sms, bool per_token) { return choose_tile_tokens(M, T, sms, per_token); }
 
 int prefill_sums_variant() {
     if (!g_tc.sums) return -1;

@@ -1,32 +1,34 @@
-"""Prefill GEMM (csrc/gemm_tc.cu) in the modes whose tiles are two row blocks high: every tile width, with
-an odd number of row blocks (the last tile's second one does not exist), a ragged last token block and
-more steps than step slots. The operands are e4m3 numbers that stand for the codes exactly, an int8
-activation as the sum of two: the codes here are drawn from all their values, -128 and -8 too, and
-the weights have every zero point. Every output word is compared with the oracle; all sums up to the
-promote are exact integers, so no tolerance is needed."""
+"""Prefill GEMM (csrc/gemm_tc.cu) in the modes whose promote reads a scale per token and group: every tile width
+of two row blocks, with an odd number of row blocks (the last tile's second one does not exist), and the one of a
+single row block, with a ragged last token block and more steps than step slots. The operands are e4m3
+numbers that stand for the codes exactly, an int8 activation as the sum of two: the codes here are drawn from all
+their values, -128 and -8 too, and the weights have every zero point. Every output word is compared with the
+oracle; all sums up to the promote are exact integers, so no tolerance is needed."""
 import numpy as np
 import pytest
 
 # tokens a tile -> rows, tokens
 SIZES = {32: (384, 688), 48: (7552, 136), 64: (9600, 152), 80: (9600, 200), 96: (9600, 248), 112: (9600, 296),
-         128: (9600, 344)}
-K = 1088                # 17 steps on 6 to 8 slots
+         128: (9600, 344), 256: (4736, 1000)}
+K = 1088                # 17 steps on 4 to 8 slots
 SMS = 148
-
-
-def tile_tokens(M, T):
-    """The kernel's choice: rounds of tiles of 256 rows over the SMs, a round counted as tokens + 26."""
-    def cost(tn):
-        tiles = (M + 255) // 256 * ((T + tn - 1) // tn)
-        return (tiles + SMS - 1) // SMS * (tn + 26)
-    return min(range(128, 31, -16), key=cost)
 
 
 @pytest.mark.parametrize("width", SIZES)
 def test_sizes_reach_every_width(lib_host, width):
     M, T = SIZES[width]
-    assert tile_tokens(M, T) == width and M % 256 == 128 and T % width
+    assert lib_host.qwn_dbg_prefill_tile(M, T, 0, SMS) == width and M % 256 == 128 and T % width
     assert lib_host.qwn_choose_gemm_splits(M // 16, T // 8, K // 32) == 1
+
+
+def test_widths_of_ordinary_calls(lib_host):
+    tile = lib_host.qwn_dbg_prefill_tile
+    assert [tile(M, T, 0, SMS) for M, T in ((10240, 136), (5120, 1000), (17408, 4096))] == [48, 80, 128]
+    # one round of 256 tokens x 128 rows where pairs of row blocks need two, pairs where they need one as well
+    assert tile(4736, 1024, 0, SMS) == tile(1664, 2728, 0, SMS) == tile(1152, 4056, 0, SMS) == 256
+    assert tile(9472, 512, 0, SMS) == 128
+    assert {tile(M, T, 1, SMS) for M in (128, 5120, 17408) for T in (128, 256, 1000, 2048)} <= {128, 192, 256}
+    assert tile(100, 128, 0, SMS) == tile(128, 120, 0, SMS) == tile(128, 132, 0, SMS) == -1
 
 
 @pytest.fixture(scope="module")
