@@ -595,13 +595,13 @@ __device__ __forceinline__ void tc_gemm(const TcParams &p, const unsigned gen) {
                 tc_fence_before();
                 __syncwarp();
                 if (kOneArrive) {
-                    mbar_arrive_if(lane == 0 ? abar + NB * 8 : ebar /* empty0 + ss * 8 */, lane < 2);
+                    mbar_arrive_if(lane == 0 ? abar + NB * 8 : ebar, lane < 2);
                 } else {
                     mbar_arrive_if(abar + NB * 8, lane == 0);
                     if (kReadsSlot && g == 1) {
                         fence_proxy_async_smem();
                         __syncwarp();
-                        mbar_arrive_if(ebar /* empty0 + ss * 8 */, lane == 0);
+                        mbar_arrive_if(ebar, lane == 0);
                     }
                 }
                 tcol += G::kAccCols;

@@ -1,12 +1,13 @@
-"""Prefill GEMM (csrc/gemm_tc.cu): every tile width it chooses between, and a caller whose code sums
-are not the sums of its codes.
+"""Prefill GEMM (csrc/gemm_tc.cu): the tile widths of the per-token mode, the other modes at the same sizes, and a
+caller whose code sums are not the sums of its codes.
 
-The kernel takes 128, 192 or 256 tokens a tile, by the rounds that M / 128 row blocks x token
+With per-token scales the kernel takes 128, 192 or 256 tokens a tile, by the rounds that M / 128 row blocks x token
 blocks make on 148 SMs; the sizes below select each of them, with a ragged last block, a full one
-and more than one round of tiles. A tile is K / 64 steps; the step slots (6, 5 and 4 at the three
-widths) and the accumulator buffers are used in turn, so REFILL goes through every slot at least
-twice, with odd step counts, within one tile and from tile to tile. Zero points are taken off the weights before the dot, so that
-z * asum enters as z * sum(codes); an asum that is something else takes a kernel of its own. Every
+and more than one round of tiles. (The other modes take tiles of their own at these sizes; test_prefill_widths.py goes
+through those.) A tile is K / 64 steps; the step slots (8, 6 and 5 at the three widths per token, 4 to 8 in the other
+modes) and the accumulator buffers are used in turn, so REFILL has more steps than slots, odd step counts, within one tile and
+from tile to tile. Zero points are taken off the weights before the dot, so that
+z * asum enters as z * sum(codes); an asum that is something else takes a form of its own. Every
 output word is compared with the oracle, which reads asum as given: all terms up to the promote are
 integers below 2^24 in either association, so no tolerance is needed."""
 import os
@@ -17,7 +18,7 @@ import pytest
 
 SIZES = [
     (5120, 128, 136),      # few row blocks
-    (9472, 128, 248),      # 128 a tile, exactly one round
+    (9472, 128, 248),      # 128 a tile per token, exactly one round
     (10240, 128, 136),     # 192 a tile, one ragged block
     (17408, 128, 256),     # 256 a tile, one full block
     (17408, 64, 320),      # several rounds: a CTA walks from tile to tile
@@ -28,11 +29,11 @@ ONE_ROW_BLOCK = {
     "other": [(128, 64, 136), (128, 192, 1000)],
 }
 REFILL = [
-    (1024, 1600, 256),     # 128 a tile, 25 steps: every slot refilled four times
+    (1024, 1600, 256),     # 128 a tile, 25 steps: every slot refilled three times
     (19200, 320, 128),     # 128 a tile, two tiles of 5 steps on a CTA
-    (9600, 1088, 136),     # 192 a tile, 17 steps on 5 slots
+    (9600, 1088, 136),     # 192 a tile, 17 steps on 6 slots
     (20480, 320, 136),     # 192 a tile, two tiles of 5 steps on a CTA
-    (9600, 832, 200),      # 256 a tile, 13 steps on 4 slots
+    (9600, 832, 200),      # 256 a tile, 13 steps on 5 slots
     (28544, 320, 200),     # 256 a tile, two tiles of 5 steps on a CTA
 ]
 MODES = ["block_k32", "block_k64", "token_k32", "token_k64", "w4a4"]
@@ -43,19 +44,39 @@ def _buf(pkg, a):
     return pkg.DevBuf.from_numpy(np.ascontiguousarray(a))
 
 
+def _unfenced_releases(source):
+    """Releases of a step slot in the workers (arrives on `ebar`) that no proxy fence of their own branch precedes, behind
+    the last read of the slot; and the number of releases."""
+    text = re.sub(r"//[^\n]*|/\*.*?\*/", "", source, flags=re.S)
+    workers = text[text.index("if (warp < kWorkWarps)"):text.index("reg_dealloc<kRoleRegs>();")]
+    reads = [m.end() for m in re.finditer(r"\bchunk\(std::integral_constant|\blds_\w+\(", workers)]
+    bad, releases = [], list(re.finditer(r"mbar_arrive_if\([^;]*\bebar\b[^;]*;", workers))
+    for m in releases:
+        behind = workers[max(r for r in reads if r < m.start()):m.start()]
+        if max(reads) > m.start():
+            bad.append(m.group())                      # a read behind the release
+        elif "abar" in m.group():                      # one arrive for both barriers: a group per step
+            if not re.search(r"if \(kOneArrive\) fence_proxy_async_smem\(\);.*__syncwarp\(\);", behind, re.S):
+                bad.append(m.group())
+        else:                                          # the innermost block of the release
+            if not re.search(r"fence_proxy_async_smem\(\);\s*__syncwarp\(\);\s*$", behind[behind.rindex("{"):]):
+                bad.append(m.group())
+    return bad, len(releases)
+
+
 def test_slots_are_released_behind_a_proxy_fence():
     """The next bulk copy into a slot writes through the async proxy, so the workers' reads of it are
     fenced before the arrive that allows it (read from the source: a copy that comes too early shows
-    only in the timing of some runs)."""
+    only in the timing of some runs). Without either fence the check fails."""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     with open(os.path.join(root, "knivesysl-xe_b200", "csrc", "gemm_tc.cu")) as f:
-        text = re.sub(r"//[^\n]*", "", f.read())
-    workers = text[text.index("if (warp < kWorkWarps)"):text.index("reg_dealloc<kRoleRegs>();")]
-    releases = [m.start() for m in re.finditer(r"mbar_arrive_if\([^;]*empty0 \+ ss", workers)]
-    assert releases
-    for at in releases:
-        last_read = max(workers.rfind("= sv[", 0, at), workers.rfind("sv_base +", 0, at))
-        assert "fence_proxy_async_smem();" in workers[last_read:at]
+        source = f.read()
+    assert _unfenced_releases(source) == ([], 2)
+    fences = [m.span() for m in re.finditer(r"fence_proxy_async_smem\(\);", source)]
+    assert len(fences) == 2
+    for a, b in fences:
+        bad, n = _unfenced_releases(source[:a] + ";" + source[b:])
+        assert n == 2 and len(bad) == 1
 
 
 @pytest.mark.gpu
