@@ -428,21 +428,30 @@ def test_w8a8_tier(orc):
     assert orc.gemm_w8a8(c8, s8, M, K, aq, as_, 12)[0] == -2
 
 
-def test_fp16_operands_keep_the_integer_dot_exact():
-    """Why the prefill kernel may run an integer dot on the f16 tensor pipe: 4-bit codes and int8
-    activations are fp16 values, each product (|.| <= 8 * 127) and every partial sum of a K64 group
-    (|.| <= 64 * 8 * 127 < 2^24) is an integer that fp32 holds exactly, so accumulating the fp16
-    products in fp32 in ANY order gives (float)d. Checked on extreme and on random operands."""
+def test_e4m3_operands_keep_the_integer_dot_exact():
+    """Why the prefill kernel may run an integer dot on the e4m3 tensor pipe: a 4-bit code less its zero point
+    (-15..15) is an e4m3 value, and an int8 code is the sum of two, its low nibble and the multiple of 16 that is
+    left. Each product and every partial sum of a K64 group (|.| <= 64 * 15 * 128 = 122880 < 2^24) is an integer that
+    fp32 holds exactly, so accumulating the products in fp32 in ANY order gives (float)d. Checked on extreme and on
+    random operands."""
+    # the finite values of e4m3: sign, 4 exponent bits (bias 7, 0: subnormal), 3 mantissa bits; 0x7F is NaN
+    bits = np.arange(0x7F)
+    e, m = bits >> 3, bits & 7
+    e4m3 = set(np.where(e == 0, m / 8.0 * 2.0 ** -6, (1 + m / 8.0) * 2.0 ** (e - 7.0)).tolist())
+    e4m3 |= {-v for v in e4m3}
+    codes = np.arange(-128, 128)
+    low = codes & 15
+    high = codes - low
+    assert set(range(-15, 16)) | set(low.tolist()) | set(high.tolist()) <= e4m3
+    assert high.min() == -128 and high.max() == 112 and (high % 16 == 0).all()
     rng = np.random.default_rng(3)
-    cases = [(np.full(64, -8), np.full(64, -127)), (np.full(64, -8), np.full(64, 127)),
-             (np.full(64, 7), np.full(64, 127))]
-    cases += [(rng.integers(-8, 8, 64), rng.integers(-127, 128, 64)) for _ in range(200)]
-    for q, a in cases:
-        qh, ah = q.astype(np.float16), a.astype(np.float16)
-        assert np.array_equal(qh.astype(np.int64), q) and np.array_equal(ah.astype(np.int64), a)
-        d = int(np.dot(q.astype(np.int64), a.astype(np.int64)))
-        prod = qh.astype(np.float32) * ah.astype(np.float32)
-        for order in (np.arange(64), np.arange(64)[::-1], rng.permutation(64)):
+    cases = [(np.full(64, w), np.full(64, a)) for w in (-15, 15, 1) for a in (-128, 127, 1)]
+    cases += [(rng.integers(-15, 16, 64), rng.integers(-128, 128, 64)) for _ in range(200)]
+    for w, a in cases:
+        d = int(np.dot(w.astype(np.int64), a.astype(np.int64)))
+        a_low = a & 15
+        prod = np.concatenate([w * (a - a_low), w * a_low]).astype(np.float32)
+        for order in (np.arange(128), np.arange(128)[::-1], rng.permutation(128)):
             acc = np.float32(0.0)
             for k in order:
                 acc = np.float32(acc + prod[k])

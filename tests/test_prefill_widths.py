@@ -74,3 +74,50 @@ def test_all_codes_at_every_width(lib, pkg, orc, wl, width, mode, wrong_sums):
         lib.tq_sync()
         assert lib.tq_last_error() == 0
         assert y.to_numpy(np.float32).tobytes() == np.ascontiguousarray(want, dtype=np.float32).tobytes()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["block_k32", "block_k64", "token_k32", "token_k64", "w4a4"])
+def test_largest_sums_are_exact(lib, pkg, mode):
+    """The largest sums that a group can have (weights of -15 or 15, activations of -128, in 4 bits -8) with a few terms of
+    1 among them: an accumulator that dropped a bit of theirs would show, for with scales of 1 every result is an
+    integer below 2^24."""
+    M, K, T = 2048, 192, 136
+    int4, ksh = mode == "w4a4", int(not mode.endswith("k32"))
+    if mode.startswith("block"):
+        assert pkg.load().qwn_choose_gemm_splits(M // 16, T // 8, K // 32) == 1
+    rows, toks, ks = np.arange(M)[:, None], np.arange(T)[:, None], np.arange(K)[None, :]
+    # even rows: zero point 7, codes -8 (-15) and 6 (-1); odd rows: zero point -8, codes 7 (15) and -7 (1)
+    z = np.where(rows % 2 == 0, 7, -8)
+    one_w = (rows + ks) % 61 == 0
+    q = np.where(rows % 2 == 0, np.where(one_w, 6, -8), np.where(one_w, -7, 7))
+    one_a = (3 * toks + ks) % 37 == 0
+    a = np.where(one_a, np.where(ks % 2 == 0, 1, -1), -8 if int4 else -128)
+    want = a.astype(np.int64) @ (q - z).astype(np.int64).T
+    assert np.abs(want).max() > K * 15 * (8 if int4 else 128) * 0.9 and np.abs(want).max() < 2 ** 24
+    n = (q & 15).astype(np.uint8).reshape(M // 16, 16, K // 32, 16, 2).transpose(0, 2, 1, 3, 4)
+    codes = n[..., 0] | (n[..., 1] << 4)
+    grp = 64 if ksh else 32
+    word = (0x3C00 | (z & 15)).astype(np.uint16)          # fp16 1.0 with the zero point in its low nibble
+    scales = np.broadcast_to(word.reshape(M // 16, 1, 16), (M // 16, K // grp, 16))
+    w = pkg.PackedWeight(codes, np.ascontiguousarray(scales), M, K, k64=bool(ksh))
+    blk = 64 if int4 else 32
+    ab = a.reshape(T, K // blk, blk).transpose(1, 0, 2)
+    sm = ab.sum(2).astype(np.int32)
+    if int4:
+        nib = (ab & 15).astype(np.uint8).reshape(K // 64, T, 32, 2)
+        staged = nib[..., 0] | (nib[..., 1] << 4)
+    else:
+        staged = ab.astype(np.int8)
+    dq, ds, dsm, dat = (pkg.DevBuf.from_numpy(np.ascontiguousarray(v))
+                        for v in (staged, np.ones(sm.size, np.float32), sm, np.ones(T, np.float32)))
+    y = pkg.DevBuf(T * M * 4)
+    if int4:
+        assert lib.qwn_x_gemm_w4a4(w.ref, dq.ptr, ds.ptr, dsm.ptr, y.ptr, T) == 0
+    elif mode.startswith("token"):
+        assert lib.qwn_x_gemm_w4a8_pertoken(w.ref, dq.ptr, dat.ptr, dsm.ptr, y.ptr, T, 0) == 0
+    else:
+        assert lib.qwn_x_gemm_w4a8(w.ref, dq.ptr, ds.ptr, dsm.ptr, y.ptr, T, None, 0) == 0
+    lib.tq_sync()
+    assert lib.tq_last_error() == 0
+    assert np.array_equal(y.to_numpy(np.float32).reshape(T, M), want.astype(np.float32))
