@@ -313,8 +313,9 @@ gemm_w4a8_batch_kernel(const GemmArgs a, const BatchArgs b, float *__restrict__ 
 // a penalty where that is this one and it loses against the other, over 3500 calls drawn from 128 to 17408 rows,
 // one to four weights, K 512 to 17408, both scale groups and 16 to 64 tokens, every plan measured. There the calls run
 // in 0.80 of the other kernel's time, 0.2 % above the best plan of each; 15 are more than 3 % behind the other kernel, two more
-// than 8 %, and of 440 calls that the constants had not seen four, the worst by 9 %. Counting a warp's instructions alone, without the sums of the splits and the rounds, left 243 of them more
-// than 3 % behind, one by 46 % (912 x 6464 K64, 40 tokens: 13.3 us against 9.2).
+// than 8 %, and of 440 calls that the constants had not seen nine, the worst by 9 % (960 x 2528, 24 tokens: 6.9 us
+// against 6.3). Counting a warp's instructions alone, without the sums of the splits and the rounds, left 243 of the
+// 3500 more than 3 % behind, one by 46 % (912 x 6464 K64, 40 tokens: 13.3 us against 9.2).
 namespace {
 
 constexpr double kLead = 1.045;

@@ -28,8 +28,8 @@
 //
 // A CTA (20 warps, one per SM, persistent over tiles) runs three roles connected by
 // mbarriers (step slots in shared memory, accumulator buffers in the 512 columns of TMEM):
-//  * one thread starts the bulk (TMA) copies of a step: 8 KiB of weights a row block and the activations of
-//    the tile's tokens, each contiguous in its image;
+//  * one thread starts the bulk (TMA) copies of a step: 8 KiB of weights a row block, with 1 KiB of their scales unless
+//    the activation scales are per token, and the activations of the tile's tokens, each contiguous in its image;
 //  * two MMA threads (in two warps): the tcgen05.mma of a k-tile into the
 //    promote group's accumulator buffer (the first one overwrites it), then tcgen05.commit;
 //  * workers (16 warps): thread = a row of every row block x a quarter of the tile's tokens. Per promote group:
@@ -81,7 +81,8 @@ constexpr int kThreads = (kWorkWarps + 4) * 32;
 // A launch with 20 warps gives every thread 96 registers (61440 of the SM's); the workers of the
 // widest tiles, whose 64 accumulators and loaded columns do not fit in that, take 104 and the other
 // four warps keep 64: 512 * 104 + 128 * 64 = 61440, exactly what the launch holds. (112 and 32: the
-// MMA and copy threads spill, and per-token prefill of 4096 tokens took 0.80 instead of 0.69 ms.)
+// MMA and copy threads spill, and per-token prefill of 4096 tokens took 0.80 instead of 0.69 ms.) Of the forms that
+// apply no sums only the 256-token tile in block mode spills (36 bytes); with sums the widest ones do (up to 148).
 constexpr int kLaunchRegs = 96, kWorkRegs = 104, kRoleRegs = 64;
 static_assert(kWorkWarps * 32 * kWorkRegs + 4 * 32 * kRoleRegs <= kThreads * kLaunchRegs,
               "the register split must not exceed what the launch holds");
@@ -139,8 +140,8 @@ struct SumsState {
     unsigned arrived;            // CTAs of the last kernel that have read the words
     unsigned last;               // the call before: did it apply the sums?
 };
-// Stamps *word unless it is stamped already: a store by every CTA costs far more than the look (136
-// tokens on 10240 x 5120 with zero points: 167 us instead of 113, 258 with a store by every warp).
+// Stamps *word unless it is stamped already: a store by every CTA costs far more than the look (54 us of a call with
+// 1184 CTAs of the pre-pass, 145 with a store by every warp; 10240 x 5120, 136 tokens, in the version with fp16 operands).
 __device__ __forceinline__ void stamp(unsigned *word, unsigned gen) {
     if (__ldcg(word) != gen) *word = gen;
 }
@@ -148,7 +149,7 @@ __device__ __forceinline__ void stamp(unsigned *word, unsigned gen) {
 __device__ __forceinline__ unsigned next_generation(unsigned g) { return g + 1 ? g + 1 : 1; }
 
 struct TcParams {
-    const uint8_t *wimg;     // per (128-row block, k-tile): kABytes of e4m3 weights in operand layout
+    const uint8_t *wimg;     // per (128-row block, step): kWImgStep bytes, the e4m3 weights of both k-tiles, then their scales
     const uint16_t *scales;
     const uint8_t *img;      // per (TN-token block, step): kImgStep bytes (see the pre-pass)
     void *y;
@@ -209,13 +210,13 @@ struct PrepassArgs {
 
 // Pre-pass: both operands of the GEMM into the layout its tiles copy, in one launch.
 //  * Weights (the first wblocks CTAs): packed codes [row group][k-tile][16 rows][16 B] -> per
-//    (128-row block, k-tile) the kABytes of e4m3 values q - z in the operand layout (row groups
-//    of 8 are kSbo apart, a row's two 16-byte K-chunks kLbo apart). With the zero point taken
-//    off here the tensor core's dot is d - z * sum(codes) itself (integers below 2^18, exact), so
+//    (128-row block, step) twice the kABytes of e4m3 values q - z of a k-tile in the operand layout (row groups
+//    of 8 are kSbo apart, a row's two 16-byte K-chunks kLbo apart), then twice the rows' scales as fp32. With the zero point taken
+//    off here the tensor core's dot is d - z * sum(codes) itself (integers below 2^17, exact), so
 //    the GEMM promotes asymmetric weights like symmetric ones. A thread expands one row of one
 //    k-tile, by a table of the 16 codes for the row's zero point; 8 consecutive lanes write 128
-//    contiguous bytes per chunk. 2 bytes out per packed byte: 89 MB for 17408 x 5120, written and read
-//    once per call.
+//    contiguous bytes per chunk. 2.25 bytes out per packed byte: 100 MB for 17408 x 5120, written once per call
+//    and read by every token block's tiles, from L2 where they run together.
 //  * Activations: the caller's staging -> per (TN-token block, step of two k-tiles) the e4m3
 //    codes of k-tile 0 then 1 as [TN / 8][2 K-chunks][8 tokens][16 B], of an int8 code first the part that is
 //    a multiple of 16, then the low nibbles; as[2][TN], and (sum of the codes - asum)[2][TN], 0
@@ -794,7 +795,7 @@ __global__ void __maxnreg__(kLaunchRegs) gemm_w4a8_tc_kernel(const TcParams p) {
 struct TcScratch {
     uint8_t *img = nullptr;
     size_t img_bytes = 0;
-    uint8_t *wimg = nullptr;      // e4m3 image of the call's weight (2 bytes per packed byte)
+    uint8_t *wimg = nullptr;      // e4m3 image of the call's weight, with its scales (2.25 bytes per packed byte)
     size_t wimg_bytes = 0;
     SumsState *sums = nullptr;
 } g_tc;
