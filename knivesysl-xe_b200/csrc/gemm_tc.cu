@@ -81,8 +81,9 @@ constexpr int kThreads = (kWorkWarps + 4) * 32;
 // A launch with 20 warps gives every thread 96 registers (61440 of the SM's); the workers of the
 // widest tiles, whose 64 accumulators and loaded columns do not fit in that, take 104 and the other
 // four warps keep 64: 512 * 104 + 128 * 64 = 61440, exactly what the launch holds. (112 and 32: the
-// MMA and copy threads spill, and per-token prefill of 4096 tokens took 0.80 instead of 0.69 ms.) Of the forms that
-// apply no sums only the 256-token tile in block mode spills (36 bytes); with sums the widest ones do (up to 148).
+// MMA and copy threads spill, and per-token prefill of 4096 tokens took 0.80 instead of 0.69 ms.) No form
+// without sums spills but the 80-token tile in W4A4 (24 bytes, both forms in one kernel); with sums the widest ones do (up to
+// 148).
 constexpr int kLaunchRegs = 96, kWorkRegs = 104, kRoleRegs = 64;
 static_assert(kWorkWarps * 32 * kWorkRegs + 4 * 32 * kRoleRegs <= kThreads * kLaunchRegs,
               "the register split must not exceed what the launch holds");
@@ -546,8 +547,10 @@ __device__ __forceinline__ void tc_gemm(const TcParams &p, const unsigned gen) {
                         }
                         float w[4] = {ws[h], ws[h], ws[h], ws[h]};
                         if constexpr (!PERTOK) {
-                            unpack2(mul2(ws2[h], as[j].x), w[0], w[1]);        // ws * as, rounded once
-                            unpack2(mul2(ws2[h], as[j].y), w[2], w[3]);
+                            // one row block: read here, not ahead of the TMEM wait, where they spill (119 against 114 us)
+                            const ulonglong2 a4 = R == 1 ? lds_pairs(at + 16 * j) : as[j];
+                            unpack2(mul2(ws2[h], a4.x), w[0], w[1]);           // ws * as, rounded once
+                            unpack2(mul2(ws2[h], a4.y), w[2], w[3]);
                         }
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
@@ -560,14 +563,9 @@ __device__ __forceinline__ void tc_gemm(const TcParams &p, const unsigned gen) {
                     const uint32_t at = svg + col * 4;
                     if constexpr (R == 1) {
                         uint32_t d[N];
-                        ulonglong2 as[N / 4];
                         tmem_ldn(tcol + col, d);
-                        if constexpr (!PERTOK) {
-#pragma unroll
-                            for (int j = 0; j < N / 4; ++j) as[j] = lds_pairs(at + 16 * j);
-                        }
                         tmem_wait_ldn(d);
-                        promote(d, as, at, 0, i0);
+                        promote(d, nullptr, at, 0, i0);
                     } else {
                         uint32_t d0[N], d1[N];
                         ulonglong2 as[N / 4];
@@ -853,9 +851,9 @@ void launch_width(const TcParams &p, int TN, int sms) {
 // width need: 136 tokens on 10240 rows are one round of 48 (us of the whole call: 67; 64 tokens: 81, 128: 122), 1000 on
 // 5120 rows two of 80 (485; 96: 535, 128: 680). With one constant for both scale groups, and one for block mode and W4A4,
 // the choice is within 1 % of the fastest width over twelve shapes in all modes. In block and 4-bit mode there is one tile of a single row block too, 256 tokens wide, for calls that it takes
-// in one round and pairs do not, an odd number of row blocks most of all (4736 x 5120, 37 of them, 1024 tokens: 119
-// against 138 us in two rounds of 80, W4A4 67 against 86); 124 against 112 us where both are one round, hence its 82 units less
-// than the 256 tokens (9472 x 5120, 512 tokens).
+// in one round and pairs do not, an odd number of row blocks most of all (4736 x 5120, 37 of them, 1024 tokens: 114
+// against 138 us in two rounds of 80, W4A4 68 against 86). Where both are one round it is the slower one (9472 x 5120, 512
+// tokens, 112 us in pairs), hence 256 - 82 units.
 int choose_tile_tokens(int M, int T, int sms, bool per_token) {
     const int rows = (per_token ? 1 : 2) * kTM, widest = per_token ? 256 : 128, step = per_token ? 64 : 16;
     int best = 0;
